@@ -27,6 +27,24 @@ __device__ __forceinline__ void mbar_init_fence() {
 __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
     asm volatile("mbarrier.arrive.shared.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// the same for the lanes with `pred` set, without a branch
+__device__ __forceinline__ void mbar_arrive_if(unsigned long long* bar, bool pred) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %1, 0;\n @p mbarrier.arrive.shared.b64 _, [%0];\n}\n" ::"r"(
+                     smem_u32(bar)),
+                 "r"((int)pred)
+                 : "memory");
+}
+// shared-memory store for the lanes with `pred` set, without a branch.  No memory
+// clobber: it is ordered with other asm volatile statements only, so loads that do
+// not read the location can be scheduled around it.
+__device__ __forceinline__ void st_shared_if(double* dst, double v, bool pred) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p st.shared.f64 [%0], %1;\n}\n" ::"r"(smem_u32(dst)), "d"(v),
+                 "r"((int)pred));
+}
+__device__ __forceinline__ void st_shared_if(float* dst, float v, bool pred) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p st.shared.f32 [%0], %1;\n}\n" ::"r"(smem_u32(dst)), "f"(v),
+                 "r"((int)pred));
+}
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }

@@ -462,14 +462,15 @@ struct Seq {
     }
     void sweeps() {
         if (c->nsf == 0) return;  // a rank without planes
-        launch_sweep_reset(s, c->d_progress, c->d_tickets, c->nsf, c->nsb);
         if (c->use_sw3) {
             n += timed(c, SCFD_K_PACK, [&] { return launch_wave(v, s, c->sw3, 0, 0); });
             n += timed(c, SCFD_K_SWEEP_FWD, [&] { return launch_wave(v, s, c->sw3, 1, 0); });
             n += timed(c, SCFD_K_SWEEP_BWD, [&] { return launch_wave(v, s, c->sw3, 2, 0); });
-            if (c->d.scheme == SCFD_SCHEME_NR) n += timed(c, SCFD_K_UPDATE, [&] { return launch_wave(v, s, c->sw3, 4, 0); });
+            if (dual_time_scheme(c->d.scheme))
+                n += timed(c, SCFD_K_UPDATE, [&] { return launch_wave(v, s, c->sw3, 4, 0); });
             return;
         }
+        launch_sweep_reset(s, c->d_progress, c->d_tickets, c->nsf, c->nsb);
         n += timed(c, SCFD_K_SWEEP_FWD, [&] {
             return launch_sweep(v, s, 0, c->d_xfer, c->d_progress, c->d_partials, c->d_tickets, c->nsf, c->nsb,
                                 c->d_strips_f, c->d_strips_b);
@@ -479,10 +480,10 @@ struct Seq {
                                 c->d_strips_f, c->d_strips_b);
         });
     }
-    // the (res, omega) partials of the last backward sweep: per pack block
-    // (k_omega) on the wavefront path, per strip on the one-warp-per-strip path
-    const double* partials() const { return c->use_sw3 ? c->sw3.partials : c->d_partials; }
-    int nstrips() const { return c->use_sw3 ? c->sw3.nstrips : c->nsb; }
+    // (res, omega) of the last backward sweep: one pair (k_omega's total) on the
+    // wavefront path, partials per strip on the one-warp-per-strip path
+    const double* partials() const { return c->use_sw3 ? c->sw3.partials + 2 * c->sw3.nblk : c->d_partials; }
+    int nstrips() const { return c->use_sw3 ? 1 : c->nsb; }
     // q update after the sweeps: NR relaxes with the omega reduced from
     // `part` (nparts strip partials); LU-SGS (inner = 1) adds Dq
     void update(int inner, const double* part, int nparts) {
@@ -490,7 +491,6 @@ struct Seq {
             if (c->nsf == 0) return;
             Wave w3 = c->sw3;
             w3.partials = const_cast<double*>(part);
-            w3.nstrips = nparts;
             n += timed(c, SCFD_K_UPDATE, [&] { return launch_wave(v, s, w3, 3, inner); });
         } else if (dual_time_scheme(c->d.scheme)) {
             n += timed(c, SCFD_K_UPDATE, [&] { return launch_nr_update(v, s, part, nparts, inner); });
@@ -777,22 +777,22 @@ int scfd_commit(scfd_ctx* c) {
     // strip records for the cluster-wavefront sweeps
     // the dual and precon schemes take the generic residual and sweeps
     const bool dual = c->d.scheme == SCFD_SCHEME_DUAL || precon_scheme(c->d.scheme);
-    const WaveSizes wz = impl && !dual ? wave_sizes(nY, mixed) : WaveSizes{0, 0, 0, 0};
+    const WaveSizes wz = impl ? wave_sizes(nY, mixed, dual) : WaveSizes{0, 0, 0, 0};
     const size_t esz3 = mixed ? sizeof(float) : sizeof(double);
     const bool legacy = std::getenv("SCFD_SWEEP_LEGACY") != nullptr;
     const char* graph_env = std::getenv("SCFD_GRAPH");
     c->use_graph = !(graph_env && std::strcmp(graph_env, "0") == 0);
-    const int ncl_max = wz.xs > 0 && !legacy ? wave_max_clusters(nY, mixed) : 0;
+    const int ncl_max = wz.xs > 0 && !legacy ? wave_max_clusters(nY, mixed, dual) : 0;
     c->use_sw3 = wz.xs > 0 && !legacy && ncl_max > 0;
     std::vector<long long> step_off;
     std::vector<int> blks3, strips3, tasksf, tasksb;
     long long steps_total = 0;
     if (c->use_sw3) {
-        const int pad = wave_pad_steps(), tpc = wave_strips_per_task();
+        const int pad = wave_pad_steps(), tpc = wave_strips_per_task(), rows = wave_rows();
         int fs = 0;
         for (int pl = 0; pl < c->np; ++pl) {
             if (!c->own(pl)) continue;
-            const int ns = (c->P.nj[pl] + 31) / 32, steps = c->P.ni[pl] + 31;
+            const int ns = (c->P.nj[pl] + rows - 1) / rows, steps = c->P.ni[pl] + rows - 1;
             const int fs_plane = fs;
             for (int st3 = 0; st3 < ns; ++st3, ++fs) {
                 step_off.push_back(steps_total);
@@ -823,7 +823,7 @@ int scfd_commit(scfd_ctx* c) {
     bytes += need<DevScalars>(1);
     bytes += 2 * need<int>(2 * c->nsf);
     bytes += need<double>((size_t)c->nsf * (c->nimax + 8) * D);
-    bytes += need<int>(c->nsf + c->nsb) + need<int>(2) + need<double>(2 * std::max<size_t>(c->nsb, blks3.size() / 2));
+    bytes += need<int>(c->nsf + c->nsb) + need<int>(3) + need<double>(2 * std::max<size_t>(c->nsb, blks3.size() / 2 + 1));
     bytes += need<GhostOp>(std::max(1, c->nops)) + need<double>(std::max<size_t>(1, c->bcs.size()) * c->valstride);
     bytes += need<long long>(std::max(1, c->nexp)) + need<HaloImport>(std::max(1, c->nimp)) +
              need<double>(std::max<long long>(1, c->seg * c->nranks)) + need<double>(8);
@@ -878,8 +878,8 @@ int scfd_commit(scfd_ctx* c) {
     c->d_strips_b = carve<int>(p, 2 * c->nsb);
     c->d_xfer = carve<double>(p, (size_t)c->nsf * (c->nimax + 8) * D);
     c->d_progress = carve<int>(p, c->nsf + c->nsb);
-    c->d_tickets = carve<int>(p, 2);
-    c->d_partials = carve<double>(p, 2 * std::max<size_t>(c->nsb, blks3.size() / 2));
+    c->d_tickets = carve<int>(p, 3);
+    c->d_partials = carve<double>(p, 2 * std::max<size_t>(c->nsb, blks3.size() / 2 + 1));
     c->d_ops = carve<GhostOp>(p, std::max(1, c->nops));
     c->d_exp = carve<long long>(p, std::max(1, c->nexp));
     c->d_imp = carve<HaloImport>(p, std::max(1, c->nimp));
@@ -923,7 +923,6 @@ int scfd_commit(scfd_ctx* c) {
         w3.blk = reinterpret_cast<const int2*>(bk);
         w3.nblk = (int)blks3.size() / 2;
         w3.strips = reinterpret_cast<const int4*>(sp);
-        w3.nstrips = w3.nblk;  // k_omega's partials: one per pack block
         w3.tasks_f = reinterpret_cast<const int4*>(tf);
         w3.tasks_b = reinterpret_cast<const int4*>(tb);
         w3.ntasks = ntasks;

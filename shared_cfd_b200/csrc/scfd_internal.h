@@ -213,27 +213,27 @@ struct Wave {
     const int4* strips;         // per forward strip (plane, s, strip, 0): pack / unpack
     const int2* blk;            // pack/unpack blocks: (strip, first step)
     int nblk;
-    int nstrips;
-    const int4* tasks_f;        // tasks of up to 8 strips (plane, first strip, strips, strip 0's index)
+    const int4* tasks_f;        // tasks of up to 256 rows (plane, first strip, strips, strip 0's index)
     const int4* tasks_b;        // backward order
     int ntasks;
     int nclusters;              // clusters launched (at most ntasks)
     void* xfer;                 // per task: published hand-off columns
     long long xstride;          // elements per task
     int* progress;              // 2*ntasks
-    int* tickets;               // 2
-    double* partials;           // (res, omega) per pack block: 2*nstrips, nstrips = nblk
+    int* tickets;               // 3: the sweeps' task tickets, k_omega's finished blocks
+    double* partials;           // (res, omega) per pack block, then of all blocks: 2*(nblk + 1)
 };
 struct WaveSizes {
     int xs, cs, d4;  // elements of an X / C step block; padded hand-off column
     size_t smem;     // dynamic shared memory of the sweep kernel
 };
-WaveSizes wave_sizes(int ny, bool mixed);  // xs = 0 if the species count has no sweep
+WaveSizes wave_sizes(int ny, bool mixed, bool pre);  // xs = 0 if there is no sweep
+int wave_rows();                           // rows per strip
 int wave_pad_steps();                      // zero step blocks before and after each strip
 int wave_strips_per_task();
 int wave_handoff_chunk();                  // hand-off columns per chunk
 int wave_chunks(int ni);                   // hand-off chunks of a top row of ni columns
-int wave_max_clusters(int ny, bool mixed); // co-resident clusters of the sweep kernel (0: none)
+int wave_max_clusters(int ny, bool mixed, bool pre); // co-resident clusters of the sweep kernel (0: none)
 int launch_wave(const View& v, cudaStream_t s, const Wave& w, int what, int inner);
 int launch_nr_update(const View& v, cudaStream_t s, const double* partials, int nstrips, int inner);
 // Cells whose CHEMEQ2 interval went to DVODE: k_chem queues them (the cell, the
@@ -297,6 +297,10 @@ __host__ __device__ inline bool dual_time_scheme(int scheme) {
 // the two schemes of time_scheme/precon and time_scheme/preconLU-SGS
 __host__ __device__ inline bool precon_scheme(int scheme) {
     return scheme == SCFD_SCHEME_PRECON || scheme == SCFD_SCHEME_PRECON_LUSGS;
+}
+// the schemes whose split Jacobians carry a low-Mach preconditioner
+__host__ __device__ inline bool preconditioned_scheme(int scheme) {
+    return scheme == SCFD_SCHEME_DUAL || precon_scheme(scheme);
 }
 
 }  // namespace scfd
