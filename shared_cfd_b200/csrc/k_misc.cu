@@ -4,12 +4,12 @@
 // field used by the mixed-precision residual.
 #include <algorithm>
 
-#include "scfd_internal.h"
+#include "cell_ops.cuh"
 
 namespace scfd {
 
 __global__ void k_dt_reset(View v) {
-    v.sc->dtmin_bits = 0x7FF0000000000000ull;  // +inf
+    v.sc->dtmin_bits = kDtInf;
 }
 
 __global__ void k_set_dt(View v) {
@@ -19,22 +19,8 @@ __global__ void k_set_dt(View v) {
     double dtc = 1e300;
     if (idx < ni * nj) {
         const int i = idx % ni + 1, j = idx / ni + 1;
-        const long long N = v.ncell;
-        const long long c = cidx(v.P, p, i, j);
-        const long long cim = cidx(v.P, p, i - 1, j), cjm = cidx(v.P, p, i, j - 1);
-        const double rho = v.w[c], u = v.w[N + c], vv = v.w[2 * N + c], pr = v.w[3 * N + c];
-        const double a = sqrt(v.w[(v.D + 1) * N + c] * pr / rho);
-        double uds = 0.0, un;
-        un = v.vni[c] * u + v.vni[N + c] * vv;
-        uds = uds + (fabs(un) + a) * v.dsi[c];
-        un = v.vni[cim] * u + v.vni[N + cim] * vv;
-        uds = uds + (fabs(un) + a) * v.dsi[cim];
-        un = v.vnj[c] * u + v.vnj[N + c] * vv;
-        uds = uds + (fabs(un) + a) * v.dsj[c];
-        un = v.vnj[cjm] * u + v.vnj[N + cjm] * vv;
-        uds = uds + (fabs(un) + a) * v.dsj[cjm];
-        dtc = v.cfl * v.Vol[c] / fmax(uds, v.w[(v.D + 4) * N + c] / rho);
-        v.dt_mat[c] = dtc;
+        dtc = cell_dt(v, p, i, j);
+        v.dt_mat[cidx(v.P, p, i, j)] = dtc;
     }
     if (v.dt_mode == SCFD_DT_GLOBAL) {
         for (int o = 16; o > 0; o >>= 1) dtc = fmin(dtc, __shfl_xor_sync(0xffffffffu, dtc, o));
@@ -43,16 +29,7 @@ __global__ void k_set_dt(View v) {
     }
 }
 
-// dt_grbl and tt (global: tt = tt + dt_grbl, set_dt.f90:40-42; fixed dt likewise)
-__global__ void k_dt_final(View v) {
-    if (v.dt_mode == SCFD_DT_GLOBAL) {
-        v.sc->dt_grbl = __longlong_as_double((long long)v.sc->dtmin_bits);
-        v.sc->tt = v.sc->tt + v.sc->dt_grbl;
-    } else if (v.dt_mode == SCFD_DT_FIXED) {
-        v.sc->dt_grbl = v.dt_fixed;
-        v.sc->tt = v.sc->tt + v.sc->dt_grbl;
-    }
-}
+__global__ void k_dt_final(View v) { dt_final(v); }
 
 // dt_mat of the updated planes and, for a global dt, their minimum in
 // dtmin_bits (+inf when there is no cell)
@@ -77,8 +54,12 @@ int launch_set_dt_cells(const View& v, cudaStream_t s) {
 int launch_set_dt(const View& v, cudaStream_t s) {
     const int n = launch_set_dt_cells(v, s);
     if (v.dt_mode == SCFD_DT_LOCAL) return n;
+    return n + launch_dt_final(v, s);
+}
+
+int launch_dt_final(const View& v, cudaStream_t s) {
     k_dt_final<<<1, 1, 0, s>>>(v);
-    return n + 1;
+    return 1;
 }
 
 // Deterministic two-pass RMS of q(E) - qp(E).

@@ -56,6 +56,7 @@ __global__ void k_dt_import(View v, const double* red) {
     if (v.dt_mode == SCFD_DT_GLOBAL) {
         sc->dt_grbl = red[0];
         sc->tt = sc->tt + sc->dt_grbl;
+        sc->dtmin_bits = kDtInf;  // the minimum starts again for the next step
     } else if (v.dt_mode == SCFD_DT_FIXED) {
         sc->dt_grbl = v.dt_fixed;
         sc->tt = sc->tt + sc->dt_grbl;

@@ -7,8 +7,8 @@
 // One thread per cell; HBM traffic per cell: read q (D) + w(4), w(R) guesses,
 // write w (W), vhi (nY), DHi (nY).  The chemkin branch is FP64 compute-bound:
 // NASA-7 polynomials in the T Newton loop and the Wilke mixture sum.
+#include "cell_ops.cuh"
 #include "div_pos.cuh"
-#include "scfd_internal.h"
 
 namespace scfd {
 
@@ -116,6 +116,39 @@ __device__ int dev_calc_T(const DevChem& ch, const double* vrho, double rho, dou
     }
     mu = mu * 1e-7;
     return 0;
+}
+
+// The rest of a step's prologue for one cell, after its w is in place: the copies of q
+// and set_dt.  Whole warps call it; `in` marks the threads with a cell.  (Ghost cells
+// written here by the threads of the cells that they copy took thermo from 123 to
+// 182 us at 786 k cells and from 10 to 30 at 768: a few threads with 26 scattered
+// stores per ghost cell; their own launch takes 3 to 10.)
+__device__ __forceinline__ void prologue(const View& v, int flags, bool in, int p, int i, int j) {
+    if (flags == 0) return;
+    const long long N = v.ncell;
+    const long long c = in ? cidx(v.P, p, i, j) : 0;
+    if (in && (flags & PRO_QP)) {
+        for (int k = 0; k < v.D; ++k) {
+            if (flags & PRO_QPP) v.qpp[k * N + c] = v.qp[k * N + c];
+            v.qp[k * N + c] = v.q[k * N + c];
+        }
+    }
+    if (flags & PRO_DT) {
+        if (v.dt_mode == SCFD_DT_FIXED) {
+            if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) dt_final(v);
+            return;
+        }
+        double dtc = 1e300;
+        if (in) {
+            dtc = cell_dt(v, p, i, j);
+            v.dt_mat[c] = dtc;
+        }
+        if (v.dt_mode == SCFD_DT_GLOBAL) {
+            for (int o = 16; o > 0; o >>= 1) dtc = fmin(dtc, __shfl_xor_sync(0xffffffffu, dtc, o));
+            if ((threadIdx.x & 31) == 0 && dtc < 1e300)
+                atomicMin(&v.sc->dtmin_bits, (unsigned long long)__double_as_longlong(dtc));
+        }
+    }
 }
 
 template <int NS>
@@ -255,13 +288,7 @@ __device__ __forceinline__ int dev_calc_T_fixed(const DevChem& ch, const double*
 // measured 1.4x slower than this, k_thermo's local-memory vectors 2x slower
 // after the same rewrite.
 template <int NS>
-__global__ void __launch_bounds__(256, 2) k_thermo_fixed(View v) {
-    const int p = v.P.act[blockIdx.y];
-    const int ni = v.P.ni[p], nj = v.P.nj[p];
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= ni * nj) return;
-    const int i = idx % ni + 1, j = idx / ni + 1;
-    const long long c = cidx(v.P, p, i, j);
+__device__ __forceinline__ void thermo_fixed(const View& v, long long c) {
     const long long N = v.ncell;
     constexpr int nY = NS, D = NS + 3;
     constexpr int ig = D + 1, iht = D + 2, iR = D + 3, imu = D + 4;
@@ -303,13 +330,19 @@ __global__ void __launch_bounds__(256, 2) k_thermo_fixed(View v) {
     w[iht * N + c] = div_pos(qE + pr, rho);
 }
 
-__global__ void __launch_bounds__(256) k_thermo(View v) {
+// PRO: with a prologue (a kernel of its own: the code costs the plain launches 5 %)
+template <int NS, bool PRO>
+__global__ void __launch_bounds__(256, 2) k_thermo_fixed(View v, int flags) {
     const int p = v.P.act[blockIdx.y];
     const int ni = v.P.ni[p], nj = v.P.nj[p];
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= ni * nj) return;
+    const bool in = idx < ni * nj;
     const int i = idx % ni + 1, j = idx / ni + 1;
-    const long long c = cidx(v.P, p, i, j);
+    if (in) thermo_fixed<NS>(v, cidx(v.P, p, i, j));
+    if (PRO) prologue(v, flags, in, p, i, j);
+}
+
+__device__ __forceinline__ void thermo_any(const View& v, long long c) {
     const long long N = v.ncell;
     const int nY = v.nY, D = v.D;
     const int ig = D + 1, iht = D + 2, iR = D + 3, imu = D + 4;  // 0-based indxg.. indxMu
@@ -363,15 +396,29 @@ __global__ void __launch_bounds__(256) k_thermo(View v) {
     w[iht * N + c] = (qE + pr) / rho;
 }
 
-int launch_thermo(const View& v, cudaStream_t s, int cells_per_plane_max) {
+template <bool PRO>
+__global__ void __launch_bounds__(256) k_thermo(View v, int flags) {
+    const int p = v.P.act[blockIdx.y];
+    const int ni = v.P.ni[p], nj = v.P.nj[p];
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = idx < ni * nj;
+    const int i = idx % ni + 1, j = idx / ni + 1;
+    if (in) thermo_any(v, cidx(v.P, p, i, j));
+    if (PRO) prologue(v, flags, in, p, i, j);
+}
+
+int launch_thermo(const View& v, cudaStream_t s, int cells_per_plane_max, int prologue) {
     if (v.P.nact == 0) return 0;
     const int bs = v.thermo_block == 64 || v.thermo_block == 256 ? v.thermo_block : 128;
     dim3 grid((cells_per_plane_max + bs - 1) / bs, v.P.nact);
     // the 9-species mechanisms (the reacting benchmark's) take the unrolled kernel
-    if (v.thermo != SCFD_THERMO_IDEAL && v.chem.ns == 9 && v.nY == 9 && v.chem.nt <= 9)
-        k_thermo_fixed<9><<<grid, bs, 0, s>>>(v);
-    else
-        k_thermo<<<grid, bs, 0, s>>>(v);
+    if (v.thermo != SCFD_THERMO_IDEAL && v.chem.ns == 9 && v.nY == 9 && v.chem.nt <= 9) {
+        if (prologue) k_thermo_fixed<9, true><<<grid, bs, 0, s>>>(v, prologue);
+        else k_thermo_fixed<9, false><<<grid, bs, 0, s>>>(v, 0);
+    } else {
+        if (prologue) k_thermo<true><<<grid, bs, 0, s>>>(v, prologue);
+        else k_thermo<false><<<grid, bs, 0, s>>>(v, 0);
+    }
     return 1;
 }
 

@@ -49,6 +49,8 @@ struct scfd_ctx {
     // boundaries
     GhostOp* d_ops = nullptr;
     int nops = 0;
+    CornerOp* d_corners = nullptr;
+    int ncorners = 0;
     double* d_bcval = nullptr;
     int valstride = SCFD_BC_MAXVAL + 2;
     // cluster-wavefront sweeps over strip records (k_wave.cu)
@@ -436,9 +438,14 @@ struct Seq {
     long long n = 0;
     explicit Seq(scfd_ctx* ctx) : c(ctx), v(ctx->v), s(ctx->stream) {}
 
-    void primitive() { n += timed(c, SCFD_K_THERMO, [&] { return launch_thermo(v, s, c->cells_max); }); }
+    // the thermo kernel, with what else of the step's prologue it does (PRO_*)
+    void primitive(int flags = 0) {
+        n += timed(c, SCFD_K_THERMO, [&] { return launch_thermo(v, s, c->cells_max, flags); });
+    }
     void bc() {
-        n += timed(c, SCFD_K_BC, [&] { return launch_ghosts(v, s, c->d_ops, c->nops, c->d_bcval, c->valstride); });
+        n += timed(c, SCFD_K_BC, [&] {
+            return launch_ghosts(v, s, c->d_ops, c->nops, c->d_corners, c->ncorners, c->d_bcval, c->valstride);
+        });
         // FP32 copies of w and vhi for the generic residual kernel (the fused one
         // rounds its tile from the FP64 state itself)
         if (v.precision == SCFD_PREC_MIXED && !fused_residual(c))
@@ -448,6 +455,7 @@ struct Seq {
         n += timed(c, SCFD_K_CHEM,
                    [&] { return launch_chem_impl(v, s, c->d.chem_max_substeps, c->d_counter, c->nsm, c->dq); });
     }
+    void dtfinal() { n += timed(c, SCFD_K_DT, [&] { return launch_dt_final(v, s); }); }
     void setdt() { n += timed(c, SCFD_K_DT, [&] { return launch_set_dt(v, s); }); }
     void copyq(double* dst, const double* src) {
         const long long qbytes = sizeof(double) * (long long)c->D * c->ncell;
@@ -501,7 +509,13 @@ struct Seq {
     }
 };
 
-// the kernel sequence of one physical step
+// The kernel sequence of one physical step.  The copies of q and set_dt ride on the
+// thermo launches where nothing has to be complete in between (a sharded step,
+// scfd_dstep, exchanges there and takes the separate launches):
+//   NR, dual, precon:  thermo, dt, chemistry, then per inner iteration thermo (the first one
+//                      also qpp = qp, qp = q), ghosts, residual, sweeps, update
+//   Euler, LU-SGS:     thermo (also qp = q, dt), for a global dt its end, ghosts, residual,
+//                      sweeps, update
 int enqueue_step(scfd_ctx* c) {
     Seq q(c);
     const View& v = c->v;
@@ -510,14 +524,16 @@ int enqueue_step(scfd_ctx* c) {
         q.primitive();
         q.setdt();
         if (reactive) q.chem();
-        q.copyq(v.qpp, v.qp);
-        q.copyq(v.qp, v.q);
         for (int j = 1; j < c->d.num_internal_loop; ++j) {
-            q.primitive();
+            q.primitive(j == 1 ? PRO_QP | PRO_QPP : 0);
             q.bc();
             q.residual(RES_NR);
             q.sweeps();
             q.update(j, q.partials(), q.nstrips());
+        }
+        if (c->d.num_internal_loop <= 1) {  // no inner iteration to ride on
+            q.copyq(v.qpp, v.qp);
+            q.copyq(v.qp, v.q);
         }
         q.step_end();
     } else {
@@ -525,12 +541,10 @@ int enqueue_step(scfd_ctx* c) {
             q.primitive();
             q.setdt();
             q.chem();
-            q.copyq(v.qp, v.q);
-            q.primitive();
+            q.primitive(PRO_QP);
         } else {
-            q.copyq(v.qp, v.q);
-            q.primitive();
-            q.setdt();
+            q.primitive(PRO_QP | PRO_DT);
+            if (c->d.dt_mode == SCFD_DT_GLOBAL) q.dtfinal();
         }
         q.bc();
         if (c->d.scheme == SCFD_SCHEME_EULER) {
@@ -754,6 +768,29 @@ int scfd_commit(scfd_ctx* c) {
     c->nexp = (int)exp_cells.size();
     c->nimp = (int)imps.size();
     c->nops = (int)ops.size();
+    std::vector<CornerOp> corners;
+    {
+        std::unordered_map<long long, int> writer;
+        for (size_t k = 0; k < ops.size(); ++k) writer[ops[k].dst] = (int)k;
+        auto by = [&](long long slot) {
+            const auto it = writer.find(slot);
+            return it == writer.end() ? -1 : it->second;
+        };
+        for (int a = 0; a < c->P.nact; ++a)
+            for (int q = 0; q < 4; ++q) {
+                const int p = c->P.act[a], pi = (q & 1) ? 1 : -1, pj = (q & 2) ? 1 : -1;
+                const int i = pi < 0 ? 1 : c->P.ni[p], j = pj < 0 ? 1 : c->P.nj[p];
+                CornerOp o;
+                o.dst = cidx(c->P, p, i + pi, j + pj);
+                o.a = cidx(c->P, p, i, j);
+                o.b = cidx(c->P, p, i, j + pj);
+                o.c = cidx(c->P, p, i + pi, j);
+                o.ob = by(o.b);
+                o.oc = by(o.c);
+                corners.push_back(o);
+            }
+    }
+    c->ncorners = (int)corners.size();
     // strips for the sweeps
     std::vector<int> sf, sb;
     for (int p = 0; p < c->np; ++p) {
@@ -824,6 +861,7 @@ int scfd_commit(scfd_ctx* c) {
     bytes += 2 * need<int>(2 * c->nsf);
     bytes += need<double>((size_t)c->nsf * (c->nimax + 8) * D);
     bytes += need<int>(c->nsf + c->nsb) + need<int>(3) + need<double>(2 * std::max<size_t>(c->nsb, blks3.size() / 2 + 1));
+    bytes += need<CornerOp>(std::max(1, c->ncorners));
     bytes += need<GhostOp>(std::max(1, c->nops)) + need<double>(std::max<size_t>(1, c->bcs.size()) * c->valstride);
     bytes += need<long long>(std::max(1, c->nexp)) + need<HaloImport>(std::max(1, c->nimp)) +
              need<double>(std::max<long long>(1, c->seg * c->nranks)) + need<double>(8);
@@ -881,6 +919,7 @@ int scfd_commit(scfd_ctx* c) {
     c->d_tickets = carve<int>(p, 3);
     c->d_partials = carve<double>(p, 2 * std::max<size_t>(c->nsb, blks3.size() / 2 + 1));
     c->d_ops = carve<GhostOp>(p, std::max(1, c->nops));
+    c->d_corners = carve<CornerOp>(p, std::max(1, c->ncorners));
     c->d_exp = carve<long long>(p, std::max(1, c->nexp));
     c->d_imp = carve<HaloImport>(p, std::max(1, c->nimp));
     c->d_halo = carve<double>(p, std::max<long long>(1, c->seg * c->nranks));
@@ -944,6 +983,9 @@ int scfd_commit(scfd_ctx* c) {
     CK(up(v.vnci, g.vnci)); CK(up(v.vncj, g.vncj));
     CK(cudaMemcpyAsync(c->d_strips_f, sf.data(), sf.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->d_strips_b, sb.data(), sb.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    if (c->ncorners)
+        CK(cudaMemcpyAsync(c->d_corners, corners.data(), corners.size() * sizeof(CornerOp), cudaMemcpyHostToDevice,
+                           c->stream));
     if (c->nops)
         CK(cudaMemcpyAsync(c->d_ops, ops.data(), ops.size() * sizeof(GhostOp), cudaMemcpyHostToDevice, c->stream));
     if (c->nexp)
@@ -1080,6 +1122,7 @@ int scfd_upload(scfd_ctx* c, const double* q, const double* w, const double* vhi
     h.tt = tt;
     h.first_dual = 1;
     h.res1 = 1.0;
+    h.dtmin_bits = kDtInf;
     CK(cudaMemcpyAsync(c->d_sc, &h, sizeof(h), cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     c->uploaded = true;
@@ -1092,7 +1135,7 @@ int scfd_prepare(scfd_ctx* c, int step) {
     (void)step;
     c->launches = 0;
     c->launches += launch_thermo(c->v, c->stream, c->cells_max);
-    c->launches += launch_ghosts(c->v, c->stream, c->d_ops, c->nops, c->d_bcval, c->valstride);
+    c->launches += launch_ghosts(c->v, c->stream, c->d_ops, c->nops, c->d_corners, c->ncorners, c->d_bcval, c->valstride);
     CK(cudaGetLastError());
     int st = sync_scalars(c);
     if (st) return st;

@@ -88,6 +88,8 @@ struct DevChem {
     double rtol, atol;        // control_chem.inp tolerances (atol: DVODE only)
 };
 
+constexpr unsigned long long kDtInf = 0x7FF0000000000000ull;  // +inf: no cell's dt yet
+
 // Scalars that live on the device between kernels of one step.
 struct DevScalars {
     double dt_grbl;
@@ -95,7 +97,7 @@ struct DevScalars {
     double omega;          // omega applied by the last NR update
     double res;            // last inner residual
     double res1;           // first inner residual of the step
-    unsigned long long dtmin_bits;  // atomicMin target for the global dt
+    unsigned long long dtmin_bits;  // atomicMin target for the global dt, kDtInf between steps
     int status;            // SCFD_* code, atomicMax
     int first_dual;
     long long chem_attempts;
@@ -191,11 +193,29 @@ struct GhostOp {
     double n1, n2;   // boundary face normal (SLIP)
 };
 
+// One corner ghost cell of set_corners: 1/3 of the interior corner cell a and the ghost
+// cells above / below and beside it, each given by the op that writes it (or, where
+// none does, by its slot).
+struct CornerOp {
+    long long dst, a, b, c;
+    int ob, oc;  // ops writing b and c, -1: none
+};
+
+// What a thermo launch does for each cell besides set_w and set_thermo_prop, so that a
+// step needs no launch (and no pass over memory) of its own for it.
+enum {
+    PRO_QP = 1,   // qp = q
+    PRO_QPP = 2,  // qpp = qp (before that)
+    PRO_DT = 4    // set_dt: the cell's dt_mat, a global dt's minimum, a fixed dt and the time
+};
+
 // kernels / launchers (stream-ordered); each returns the number of launches
-int launch_thermo(const View& v, cudaStream_t s, int cells_per_plane_max);
-int launch_ghosts(const View& v, cudaStream_t s, const GhostOp* ops, int nops, const double* bcval, int valstride);
+int launch_thermo(const View& v, cudaStream_t s, int cells_per_plane_max, int prologue = 0);
+int launch_ghosts(const View& v, cudaStream_t s, const GhostOp* ops, int nops, const CornerOp* corners, int ncorners,
+                  const double* bcval, int valstride);
 int launch_ghost_ops(const View& v, cudaStream_t s, const GhostOp* ops, int nops, const double* bcval, int valstride);
 int launch_set_dt(const View& v, cudaStream_t s);
+int launch_dt_final(const View& v, cudaStream_t s);      // dt and time from the cells' minimum
 int launch_set_dt_cells(const View& v, cudaStream_t s);  // dt_mat and the local minimum only
 int launch_residual(const View& v, cudaStream_t s, int mode, bool need_coeffs);
 bool launch_residual2(const View& v, cudaStream_t s, int mode);
