@@ -9,6 +9,13 @@
 // tile plus a 2-cell halo into shared memory with coalesced loads, then
 // computes the TY(TX+1) i-faces and (TY+1)TX j-faces of the tile from shared
 // memory (about two faces per thread), then sums faces and sources per cell.
+// What bounds it: latency, of the loads first (long_scoreboard 3.7 of 9 cycles per issue
+// in FP64, 9.5 of 16 in FP32, with DRAM at a fifth of its rate).  So each phase issues all
+// its loads before it uses or stores any: a thread stages whole cells, W values in
+// flight at once, and reads q, qp, qpp of its cell before the first store; face fluxes lie
+// component-major.  786 k cells, 9 species: FP64 0.385 -> 0.301 ms, FP32 0.357 -> 0.216;
+// 197 k cells of one species FP64 (explicit) 0.035 -> 0.028 ms.  A 16x7 tile of 128 threads
+// (every round of faces full) was slower in FP64 (0.353 against 0.313 ms then).
 // The FP64 kernel stages w and T only and reads vhi through L1: its 16x8 tile
 // then takes 61 KB of shared memory and three CTAs fit on an SM (with vhi
 // staged, two), which its latency-bound faces need more than the loads.
@@ -27,16 +34,17 @@ namespace scfd {
 
 namespace {
 
-template <int TX_, int TY_, int NTH_>
+// MINB: CTAs per SM that the FP32 kernel is built for (its registers), 0: no bound
+template <int TX_, int TY_, int NTH_, int MINB_>
 struct Tile {
-    static constexpr int TX = TX_, TY = TY_, HX = TX + 4, HY = TY + 4, NTH = NTH_;
+    static constexpr int TX = TX_, TY = TY_, HX = TX + 4, HY = TY + 4, NTH = NTH_, MINB = MINB_;
     static constexpr int NFI = TY * (TX + 1), NFJ = (TY + 1) * TX;
     static_assert(NTH >= TX * TY, "one thread per cell in the sum phase");
 };
-using Tile0 = Tile<32, 8, 288>;
-using Tile1 = Tile<16, 16, 288>;
-using Tile2 = Tile<64, 4, 288>;
-using Tile3 = Tile<16, 8, 160>;
+using Tile0 = Tile<32, 8, 288, 2>;
+using Tile1 = Tile<16, 16, 288, 2>;
+using Tile2 = Tile<64, 4, 288, 0>;
+using Tile3 = Tile<16, 8, 160, 4>;
 
 template <typename RT>
 __device__ __forceinline__ RT eps_of();
@@ -50,8 +58,8 @@ struct Smem {
     RT* w;   // [W][HY][HX]
     RT* vh;  // [NY][HY][HX]
     RT* T;   // [HY][HX]
-    RT* FI;  // [NFI][D]
-    RT* FJ;  // [NFJ][D]
+    RT* FI;  // [D][NFI] (component-major: face-major stores and loads collide in 4 banks)
+    RT* FJ;  // [D][NFJ]
 };
 
 // vhi staged in shared memory (FP32); the FP64 faces read it through L1 instead,
@@ -68,7 +76,7 @@ constexpr bool kStageVh = sizeof(RT) == 4;
 // speed, gamma - 1 and positive constants.
 template <typename RT, int NY, typename TL>
 __device__ __forceinline__ void face2(const View& v, const Smem<RT>& S, int p, int i, int j, int ix, int jy, bool iface,
-                                      RT* out) {
+                                      RT* out, int os) {
     constexpr int D = NY + 3;
     constexpr int HX = TL::HX, HS = TL::HY * TL::HX;
     const RT phi = RT(v.recon == SCFD_RECON_MUSCL ? v.phi_mus : 0.0), km = RT(v.k_mus);
@@ -76,6 +84,22 @@ __device__ __forceinline__ void face2(const View& v, const Smem<RT>& S, int p, i
     // smem cell offsets along the face normal: m1, 0 (left), 1 (right), 2
     const int st = iface ? 1 : HX;
     const int c0 = jy * HX + ix;
+    const long long N = v.ncell;
+    const long long cg = cidx(v.P, p, i, j);
+    const double* vn = iface ? v.vni : v.vnj;
+    const double* gj = iface ? v.gji : v.gjj;
+    // the FP32 face has the registers to load its metrics ahead of the limiters
+    constexpr bool kAhead = sizeof(RT) == 4;
+    RT met[7];
+    if constexpr (kAhead) {
+        met[0] = RT(__ldg(vn + cg));
+        met[1] = RT(__ldg(vn + N + cg));
+        met[2] = RT(__ldg((iface ? v.dsi : v.dsj) + cg));
+        if (v.viscous) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) met[3 + e] = RT(__ldg(gj + e * N + cg));
+        }
+    }
     RT wl[NY + 6], wr[NY + 6];
 #pragma unroll
     for (int m = 0; m < NY + 6; ++m) {
@@ -91,10 +115,7 @@ __device__ __forceinline__ void face2(const View& v, const Smem<RT>& S, int p, i
         const RT dl = half * s * ((one + km * s) * Dl + (one - km * s) * Du);
         wr[m] = w1 - phi * half * dl;
     }
-    const long long N = v.ncell;
-    const long long cg = cidx(v.P, p, i, j);
-    const double* vn = iface ? v.vni : v.vnj;
-    const RT n1 = RT(__ldg(vn + cg)), n2 = RT(__ldg(vn + N + cg));
+    const RT n1 = kAhead ? met[0] : RT(__ldg(vn + cg)), n2 = kAhead ? met[1] : RT(__ldg(vn + N + cg));
     // SLAU (scheme.f90:71-153)
     RT tg[D];
     {
@@ -126,10 +147,10 @@ __device__ __forceinline__ void face2(const View& v, const Smem<RT>& S, int p, i
         tg[NY + 1] = dpp * vl + dnn * vr + pt * n2;
         tg[NY + 2] = dpp * wl[5 + NY] + dnn * wr[5 + NY];
     }
-    const RT ds = RT(__ldg((iface ? v.dsi : v.dsj) + cg));
+    const RT ds = kAhead ? met[2] : RT(__ldg((iface ? v.dsi : v.dsj) + cg));
     if (!v.viscous) {
 #pragma unroll
-        for (int k = 0; k < D; ++k) out[k] = ds * tg[k];
+        for (int k = 0; k < D; ++k) out[k * os] = ds * tg[k];
         return;
     }
     // viscous face flux (sch_viscous.f90:125-197, 214-286)
@@ -152,9 +173,8 @@ __device__ __forceinline__ void face2(const View& v, const Smem<RT>& S, int p, i
     const RT dC_u = (W_(1, p1) + W_(1, p2) - W_(1, m1) - W_(1, m2)) * q4;
     const RT dC_v = (W_(2, p1) + W_(2, p2) - W_(2, m1) - W_(2, m2)) * q4;
     const RT dC_T = (S.T[p1] + S.T[p2] - S.T[m1] - S.T[m2]) * q4;
-    const double* gj = iface ? v.gji : v.gjj;
-    const RT g11 = RT(__ldg(gj + cg)), g12 = RT(__ldg(gj + N + cg)), g21 = RT(__ldg(gj + 2 * N + cg)),
-             g22 = RT(__ldg(gj + 3 * N + cg));
+    const RT g11 = kAhead ? met[3] : RT(__ldg(gj + cg)), g12 = kAhead ? met[4] : RT(__ldg(gj + N + cg)),
+             g21 = kAhead ? met[5] : RT(__ldg(gj + 2 * N + cg)), g22 = kAhead ? met[6] : RT(__ldg(gj + 3 * N + cg));
     const RT dudxi = iface ? dN_u : dC_u, dudeta = iface ? dC_u : dN_u;
     const RT dvdxi = iface ? dN_v : dC_v, dvdeta = iface ? dC_v : dN_v;
     const RT dTdxi = iface ? dN_T : dC_T, dTdeta = iface ? dC_T : dN_T;
@@ -192,11 +212,11 @@ __device__ __forceinline__ void face2(const View& v, const Smem<RT>& S, int p, i
     tv[NY + 1] = t_xr * n1 + t_rr * n2;
     tv[NY + 2] = (u * t_xx + vv * t_xr - qx) * n1 + (u * t_xr + vv * t_rr - qr) * n2;
 #pragma unroll
-    for (int k = 0; k < D; ++k) out[k] = ds * (tg[k] - tv[k]);
+    for (int k = 0; k < D; ++k) out[k * os] = ds * (tg[k] - tv[k]);
 }
 
 template <typename RT, int NY, int MODE, typename TL>
-__global__ void __launch_bounds__(TL::NTH) k_residual2(View v) {
+__global__ void __launch_bounds__(TL::NTH, sizeof(RT) == 4 ? TL::MINB : 0) k_residual2(View v) {
     constexpr int TX = TL::TX, TY = TL::TY, HX = TL::HX, NTH = TL::NTH, NFI = TL::NFI, NFJ = TL::NFJ;
     constexpr int D = NY + 3, W = D + 5, HS = TL::HY * HX;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -248,23 +268,27 @@ __global__ void __launch_bounds__(TL::NTH) k_residual2(View v) {
             }
         }
     }
-    for (int e = tid; e < (W + NVH) * HS; e += NTH) {
-        const int comp = e / HS, rem = e - comp * HS;
-        const int jy = rem / HX, ix = rem - jy * HX;
-        const int i = i0 - 2 + ix, j = j0 - 2 + jy;
-        RT val = RT(0);
-        if (i <= ni + 2 && j <= nj + 2) {
-            const long long c = base0 + (long long)jy * pitch + ix;
-            // the FP32 tile is rounded from the FP64 state here (the values the
-            // generic kernel's FP32 copies hold)
-            val = comp < W ? RT(__ldg(v.w + comp * N + c)) : RT(__ldg(v.vhi + (comp - W) * N + c));
-        }
-        S.w[e] = val;  // S.vh follows S.w contiguously
-    }
-    __syncthreads();
+    // a thread takes whole cells of the tile, so that all their components' loads are in
+    // flight together
     for (int e = tid; e < HS; e += NTH) {
-        const RT rr = S.w[e];
-        S.T[e] = rr != RT(0) ? S.w[3 * HS + e] / rr / S.w[(D + 3) * HS + e] : RT(0);
+        const int jy = e / HX, ix = e - jy * HX;
+        const bool in = i0 - 2 + ix <= ni + 2 && j0 - 2 + jy <= nj + 2;
+        const long long c = base0 + (long long)jy * pitch + ix;
+        // the FP32 tile is rounded from the FP64 state here (the values the
+        // generic kernel's FP32 copies hold)
+        double r[W];
+#pragma unroll
+        for (int m = 0; m < W; ++m) r[m] = in ? __ldg(v.w + m * N + c) : 0.0;
+#pragma unroll
+        for (int m = 0; m < W; ++m) S.w[m * HS + e] = RT(r[m]);
+        const RT rr = RT(r[0]);
+        S.T[e] = rr != RT(0) ? RT(r[3]) / rr / RT(r[D + 3]) : RT(0);
+        if constexpr (NVH > 0) {
+#pragma unroll
+            for (int m = 0; m < NVH; ++m) r[m] = in ? __ldg(v.vhi + m * N + c) : 0.0;
+#pragma unroll
+            for (int m = 0; m < NVH; ++m) S.vh[m * HS + e] = RT(r[m]);
+        }
     }
     __syncthreads();
     // faces: i-faces f < NFI, j-faces after
@@ -272,12 +296,12 @@ __global__ void __launch_bounds__(TL::NTH) k_residual2(View v) {
         if (f < NFI) {
             const int fy = f / (TX + 1), fx = f - fy * (TX + 1);
             const int i = i0 - 1 + fx, j = j0 + fy;
-            if (i <= ni && j <= nj) face2<RT, NY, TL>(v, S, p, i, j, fx + 1, fy + 2, true, S.FI + f * D);
+            if (i <= ni && j <= nj) face2<RT, NY, TL>(v, S, p, i, j, fx + 1, fy + 2, true, S.FI + f, NFI);
         } else {
             const int g = f - NFI;
             const int fy = g / TX, fx = g - fy * TX;
             const int i = i0 + fx, j = j0 - 1 + fy;
-            if (i <= ni && j <= nj) face2<RT, NY, TL>(v, S, p, i, j, fx + 2, fy + 1, false, S.FJ + g * D);
+            if (i <= ni && j <= nj) face2<RT, NY, TL>(v, S, p, i, j, fx + 2, fy + 1, false, S.FJ + g, NFJ);
         }
     }
     __syncthreads();
@@ -307,32 +331,46 @@ __global__ void __launch_bounds__(TL::NTH) k_residual2(View v) {
             svq_my = -t_tt;
         }
     }
-    const RT* fim = S.FI + (ty * (TX + 1) + tx) * D;
-    const RT* fip = fim + D;
-    const RT* fjm = S.FJ + (ty * TX + tx) * D;
-    const RT* fjp = S.FJ + ((ty + 1) * TX + tx) * D;
+    const RT* fi = S.FI + ty * (TX + 1) + tx;  // the cell's lower faces; the upper ones 1 and TX on
+    const RT* fj = S.FJ + ty * TX + tx;
+    auto flux_sum = [&](int k) {
+        return (double)fi[k * NFI] - (double)fi[k * NFI + 1] + (double)fj[k * NFJ] - (double)fj[k * NFJ + TX];
+    };
     const double dtl = v.dt_mode == SCFD_DT_LOCAL ? v.dt_mat[c] : v.sc->dt_grbl;
     if (MODE == RES_EULER) {
         const double fct = dtl / v.Vol[c];
+        double q1[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k) q1[k] = v.qp[k * N + c];
 #pragma unroll
         for (int k = 0; k < D; ++k) {
             const double src = k == NY + 1 ? area * (sq_my + svq_my) : area * 0.0;
-            const double rhs = (double)fim[k] - (double)fip[k] + (double)fjm[k] - (double)fjp[k] + src;
-            v.q[k * N + c] = v.qp[k * N + c] + fct * rhs;
+            const double rhs = flux_sum(k) + src;
+            v.q[k * N + c] = q1[k] + fct * rhs;
         }
         return;
     }
     const double vol = v.Vol[c];
     const bool first = v.sc->first_dual != 0;
+    // all loads before the first store, so that they overlap
+    double dq[D];
+    if constexpr (MODE == RES_NR) {
+        double q0[D], q1[D], q2[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            q0[k] = v.q[k * N + c];
+            q1[k] = v.qp[k * N + c];
+            q2[k] = v.qpp[k * N + c];
+        }
+#pragma unroll
+        for (int k = 0; k < D; ++k)
+            dq[k] = first ? (q0[k] - q1[k]) / dtl : (3.0 * q0[k] - 4.0 * q1[k] + q2[k]) / (2.0 * dtl);
+    }
 #pragma unroll
     for (int k = 0; k < D; ++k) {
         const double src = k == NY + 1 ? area * (sq_my + svq_my) : area * 0.0;
-        double rhs = (double)fim[k] - (double)fip[k] + (double)fjm[k] - (double)fjp[k] + src;
-        if (MODE == RES_NR) {
-            const double qk = v.q[k * N + c], qpk = v.qp[k * N + c];
-            const double dqdt = first ? (qk - qpk) / dtl : (3.0 * qk - 4.0 * qpk + v.qpp[k * N + c]) / (2.0 * dtl);
-            rhs = rhs - vol * dqdt;
-        }
+        double rhs = flux_sum(k) + src;
+        if (MODE == RES_NR) rhs = rhs - vol * dq[k];
         v.Dq[k * N + c] = rhs;
     }
 }
