@@ -57,6 +57,8 @@
 // The backward sweep walks the same records with steps and rows reversed.
 // k_unpack applies q += omega Dq back in the cell layout.
 #include <algorithm>
+#include <map>
+#include <mutex>
 #include <type_traits>
 
 #include "async_ptx.h"
@@ -1103,7 +1105,7 @@ WaveSizes wave_sizes(int ny, bool mixed, bool pre) {
 namespace {
 
 template <typename RT, int NY, int PRE, int DIR, int Q2D>
-int max_clusters_t() {
+int query_clusters() {
     using L = WL<RT, NY, PRE>;
     if (cudaFuncSetAttribute(k_wave<RT, NY, PRE, DIR, Q2D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM) !=
         cudaSuccess)
@@ -1135,6 +1137,22 @@ int max_clusters_t() {
         cudaGetLastError();
         return 0;
     }
+    return n;
+}
+
+// The device answers the same every time; the query takes milliseconds, so a process asks
+// once per kernel and device (the attributes that it sets stay set).
+template <typename RT, int NY, int PRE, int DIR, int Q2D>
+int max_clusters_t() {
+    static std::mutex m;
+    static std::map<int, int> known;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    std::lock_guard<std::mutex> lock(m);
+    const auto it = known.find(dev);
+    if (it != known.end()) return it->second;
+    const int n = query_clusters<RT, NY, PRE, DIR, Q2D>();
+    if (n > 0) known[dev] = n;
     return n;
 }
 
