@@ -30,9 +30,9 @@
 // A task is 256 consecutive rows of one plane at most, run by one thread-block
 // cluster of 16 CTAs with two strips each.  A strip's top row is staged in its
 // CTA's shared memory; every HK columns one bulk copy moves the chunk into the
-// next strip's hand-off ring (in the same CTA or, distributed shared memory, the
-// next one), completing a transaction count on an mbarrier of the receiver, which
-// releases consumed chunks with a (remote) arrive.  A task with a successor holds
+// next CTA's hand-off ring (distributed shared memory), completing a transaction count on
+// an mbarrier of the receiver, which releases consumed chunks with a remote arrive.  From a
+// CTA's first strip to its second the top row is written into the ring directly.  A task with a successor holds
 // all its strips, so only the last strip of a cluster ever publishes to global
 // memory and the others only to the next strip.  Between tasks of one plane the
 // top row travels through global memory: a warp of the last CTA copies it
@@ -176,7 +176,7 @@ struct WL {
 // whole lines.  Block 0 also resets the sweeps' counters.
 // ---------------------------------------------------------------------------
 template <typename T, int NY, int PRE>
-__global__ void __launch_bounds__(32 * R)
+__global__ void __launch_bounds__(32 * R, 2)
 k_pack(View v, const int2* blk, const int4* strips, const long long* step_off, T* X, T* Cr, int nr_mode, int* progress,
        int nprogress, int* tickets) {
     using L = WL<T, NY, PRE>;
@@ -200,6 +200,16 @@ k_pack(View v, const int2* blk, const int4* strips, const long long* step_off, T
     const bool ok = cc >= 0 && cc < ni && j <= nj && t < ni + R - 1;
     const long long N = v.ncell;
     const long long c = ok ? cidx(v.P, p, i, j) : 0;
+    // all of the cell's values before the first barrier, so that their loads overlap (read
+    // pass by pass they took a load latency each: 14.5 us for 768 cells)
+    double xq[D], dh[NY], yy[NY];
+#pragma unroll
+    for (int k = 0; k < D; ++k) xq[k] = ok ? v.Dq[k * N + c] : 0.0;
+#pragma unroll
+    for (int k = 0; k < NY; ++k) {
+        dh[k] = ok ? v.DHi[k * N + c] : 0.0;
+        yy[k] = ok ? v.w[(4 + k) * N + c] : 0.0;
+    }
     double cm[NM * GM] = {};  // shared fields
     double u = 0.0, vv = 0.0, H = 0.0, g1 = 0.0, hvs = 0.0, al = 0.0;
     if (ok) {
@@ -244,21 +254,21 @@ k_pack(View v, const int2* blk, const int4* strips, const long long* step_off, T
             cm[CM::RQ] = 1.0 / (1.0 - aA * (-g1 * vv));
         }
         if constexpr (NY == 1) {
-            cm[CM::D0] = hvs + v.DHi[c];
+            cm[CM::D0] = hvs + dh[0];
             cm[CM::DU] = -g1 * u;
             cm[CM::DE] = g1;
             if constexpr (PRE != 0) {
                 const bool dual = v.scheme == SCFD_SCHEME_DUAL;
                 const double s2 = dual ? v.pre[N + c] : v.pre[c];
                 // p2 . p1
-                const double k0 = (hvs + v.DHi[c]) * w[4 * N + c] + g1 * (H - (u * u + vv * vv));
+                const double k0 = (hvs + dh[0]) * yy[0] + g1 * (H - (u * u + vv * vv));
                 cm[CM::K1] = 1.0 + s2 * k0;
                 cm[CM::S2] = s2;
                 cm[CM::S1] = dual ? v.pre[c] : 1.0;
                 cm[CM::S3] = dual ? v.pre[2 * N + c] : 0.0;
                 cm[CM::S4] = dual ? v.pre[3 * N + c] : 0.0;
                 cm[CM::I1] = dual ? 1.0 / v.pre[c] : 1.0;
-                cm[CM::Y0] = w[4 * N + c];
+                cm[CM::Y0] = yy[0];
                 cm[CM::U] = u;
                 cm[CM::V] = vv;
                 cm[CM::H] = H;
@@ -266,13 +276,13 @@ k_pack(View v, const int2* blk, const int4* strips, const long long* step_off, T
         }
     }
     auto xval = [&](int k) -> double {
-        return !ok || k < 0 ? 0.0 : L::SCALED ? al * v.Dq[k * N + c] : v.Dq[k * N + c];
+        return k < 0 ? 0.0 : L::SCALED ? al * xq[k < 0 ? 0 : k] : xq[k < 0 ? 0 : k];
     };
     auto dpdq = [&](int k) -> double {
-        return !ok || k < 0 ? 0.0 : k < NY ? hvs + v.DHi[k * N + c] : k == NY ? -g1 * u : k == NY + 1 ? 0.0 : g1;
+        return k < 0 ? 0.0 : k < NY ? hvs + dh[k < 0 || k >= NY ? 0 : k] : k == NY ? -g1 * u : k == NY + 1 ? 0.0 : g1;
     };
     auto prim = [&](int k) -> double {
-        return !ok || k < 0 ? 0.0 : k < NY ? v.w[(4 + k) * N + c] : k == NY ? u : k == NY + 1 ? vv : H;
+        return k < 0 ? 0.0 : k < NY ? yy[k < 0 || k >= NY ? 0 : k] : k == NY ? u : k == NY + 1 ? vv : H;
     };
     // own coefficient e of (sub, slot): NY = 1 (primitive, pA, pB, 0), else (dpdq, primitive); dpdq of
     // rho v is left to the shared DV, which follows the pressure source
@@ -580,7 +590,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kThreads, 1) k_wave
         RT *ringX, *ringC;  // [PFB][SPB][XS], [PFB][SPB][CS]
         RT *xin, *xout;     // [HS][HK][D4]: columns from the strip below; top row for the next strip
         unsigned long long *rfull, *rdone;  // record slot loaded (expect_tx + bulk copies) / read (compute warp)
-        unsigned long long* xfull;   // hand-off chunk arrived (producer's arrival + bytes)
+        unsigned long long* xfull;   // hand-off chunk arrived (bulk copy, or the first strip's top row)
         unsigned long long* pempty;  // a chunk this strip produced is consumed (or published in global memory)
         unsigned long long* hempty;  // a chunk fetched from global memory is consumed
         unsigned long long* oful;    // xout chunk written (the top row's four lanes)
@@ -614,6 +624,9 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kThreads, 1) k_wave
         const Unit q = unit_at(threadIdx.x);
         for (int k = 0; k < 2 * PFB + 3 * HS; ++k) mbar_init(&q.rfull[k], 1);
         for (int k = 0; k < HS; ++k) mbar_init(&q.oful[k], LPC);
+        // the second strip's chunks are written by the first strip's top row itself
+        if (threadIdx.x == 1)
+            for (int k = 0; k < HS; ++k) mbar_init(&q.xfull[k], LPC);
         mbar_init_fence();
     }
     if (threadIdx.x == 0) {
@@ -696,6 +709,11 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kThreads, 1) k_wave
                 rec[0].template load<DIR>(U.ringX + o * XS, U.ringC + o * CSZ, mlane, mrow);
             }
             const bool pub_any = pub_next || pub_global;
+            // the top row goes straight into the next strip's ring where that is this CTA's, else
+            // to the warp that passes it on
+            const bool direct = pub_next && unit == 0;
+            RT* const oring = direct ? Uo.xin : U.xout;
+            unsigned long long* const obar = direct ? Uo.xfull : U.oful;
             unsigned pfree = pc + 1;  // chunks before this one may be written
             // A wait splits the code that the compiler can schedule (120-180 cycles per
             // wait in a loop of 4 steps), so a slot of 8 steps has three: for the chunk of each
@@ -728,7 +746,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kThreads, 1) k_wave
                     // zero column where there is no strip)
                     const RT* const cA = has_prev ? U.xin + ((xc + g) % HS * HK + 3) * D4 + lane % LPC * K : s_zero;
                     const RT* const cB = has_prev ? U.xin + (xc + g + 1) % HS * HK * D4 + lane % LPC * K : s_zero;
-                    RT* const xo = U.xout + ps * HK * D4 + lane % LPC * K;
+                    RT* const xo = oring + ps * HK * D4 + lane % LPC * K;
 #pragma unroll
                     for (int u = 0; u < HK; ++u) {
                         const int s = h * HK + u;  // step of the slot
@@ -777,7 +795,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kThreads, 1) k_wave
                     if (bail) break;
                     // chunk J complete: on to the warp that passes it on.
                     // Columns outside 0 .. ni-1 travel as they are.
-                    mbar_arrive_if(&U.oful[ps], put);
+                    mbar_arrive_if(&obar[ps], put);
                     pc += pub ? 1u : 0u;
                 }
                 gx += (DIR == 0 ? SPB : -SPB) * XS;
@@ -833,9 +851,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kThreads, 1) k_wave
             // ------------------------------------------------------------ hand-off to the next strip
             // one bulk copy per chunk into its ring, completing the receiver's barrier
             // phase with this arrival and the copy's bytes (in either order)
-            if (lane == 0) {
-                const unsigned nrank = unit == UPC - 1 ? rank + 1 : rank;
-                const unsigned dring = mapa(Uo.xin, nrank), dfull = mapa(Uo.xfull, nrank);
+            if (lane == 0 && unit == UPC - 1) {
+                const unsigned dring = mapa(Uo.xin, rank + 1), dfull = mapa(Uo.xfull, rank + 1);
                 for (int h = 0; h < nxc; ++h) {
                     const unsigned k = pc + h, ps = k % HS;
                     if (!wait_phase(&U.oful[ps], (k / HS) & 1u, v, s_bail)) {
