@@ -16,7 +16,7 @@
 // RT is the arithmetic type of reconstruction and fluxes (double for the plain
 // path, float for the mixed path); the right-hand-side sum, the dual-time
 // defect Vol*dqdt and the update stay in double.
-#include "scfd_internal.h"
+#include "precond.cuh"
 
 namespace scfd {
 
@@ -276,65 +276,19 @@ __global__ void __launch_bounds__(NT) k_residual(View v) {
     }
     const double vol = v.Vol[c];
     const bool first = v.sc->first_dual != 0;
-    if (MODE == RES_PRECON || MODE == RES_PRECON_LUSGS) {
-        // set_ABpm of time_scheme/precon/2d (sch_precon.raw.f90:28-77, 194-197):
-        // low-Mach reference velocity, preconditioned spectral radii, the local
-        // time step (written to dt_mat: set_dqdt and alpha use it), phh of
-        // pre1 = phh (Y, u, v, H); then Dq = R + pre1 (pre2 . R) [- Vol dqdt]
-        // (time_precon_viscous.f90:18-27)
-        const double rho = v.w[c], u = v.w[N + c], vv = v.w[2 * N + c], pr = v.w[3 * N + c];
-        const double gamm = v.w[(D + 1) * N + c], H = v.w[(D + 2) * N + c];
-        const double mu = v.w[(D + 4) * N + c], dsa = v.dsci[c], dsb = v.dscj[c];
-        const double cs = sqrt(gamm * pr / rho);
-        const double unA = v.vnci[c] * u + v.vnci[N + c] * vv;
-        const double unB = v.vncj[c] * u + v.vncj[N + c] * vv;
-        const double Vs = u * u + vv * vv;
-        const double Vv = mu / rho / fmin(dsa, dsb);
-        const double Ur = fmin(fmax(Vv, sqrt(Vs)), cs);
-        const double phi = 1.0 / (Ur * Ur) - 1.0 / (cs * cs);
-        const double alp = 0.5 * (1.0 - (Ur / cs) * (Ur / cs));
-        double ud = unA * (1.0 - alp), cd = sqrt(alp * alp * (unA * unA) + Ur * Ur);
-        const double nuA = fabs(ud) + cd;
-        ud = unB * (1.0 - alp);
-        cd = sqrt(alp * alp * (unB * unB) + Ur * Ur);
-        const double nuB = fabs(ud) + cd;
-        const long long cim = cidx(v.P, p, i - 1, j), cjm = cidx(v.P, p, i, j - 1);
-        const double uds = nuA * (v.dsi[c] + v.dsi[cim]) + nuB * (v.dsj[c] + v.dsj[cjm]);
-        const double dt = v.cfl * vol / fmax(uds, mu / rho);
-        v.dt_mat[c] = dt;
-        const double phh = -1.0 / (cs * cs + 1.0 / phi);
-        const double tmp = MODE == RES_PRECON ? 3.0 * vol / (2.0 * dt) + dsa * nuA + dsb * nuB
-                                              : vol / dt + dsa * nuA + dsb * nuB;
-        v.alpha[c] = 1.0 / tmp;
-        v.nuA[c] = nuA;
-        v.nuB[c] = nuB;
-        v.pre[c] = phh;
-        const double g1 = gamm - 1.0;
+    if (MODE == RES_PRECON || MODE == RES_PRECON_LUSGS || MODE == RES_DUAL) {
         double R[kMaxSpecies + 3];
-        double t = 0.0;
         for (int k = 0; k < D; ++k) {
             const double src = k == nY + 1 ? area * (sq_my + svq_my) : area * 0.0;
             R[k] = (double)fim[k] - (double)fip[k] + (double)fjm[k] - (double)fjp[k] + src;
-            const double p2 = k < nY ? 0.5 * g1 * Vs + v.DHi[k * N + c]
-                                     : (k == nY ? -g1 * u : (k == nY + 1 ? -g1 * vv : g1));
-            t = t + p2 * R[k];
         }
-        for (int k = 0; k < D; ++k) {
-            const double p1 = k < nY ? phh * v.w[(4 + k) * N + c] : phh * (k == nY ? u : (k == nY + 1 ? vv : H));
-            double rhs = R[k] + p1 * t;
-            if (MODE == RES_PRECON) {
-                const double qk = v.q[k * N + c], qpk = v.qp[k * N + c];
-                const double dqdt = first ? (qk - qpk) / dt : (3.0 * qk - 4.0 * qpk + v.qpp[k * N + c]) / (2.0 * dt);
-                rhs = rhs - vol * dqdt;
-            }
-            v.Dq[k * N + c] = rhs;
-        }
+        precond_cell<MODE>(v, p, i, j, c, D, R, vol, dtl, first);
         return;
     }
     for (int k = 0; k < D; ++k) {
         const double src = k == nY + 1 ? area * (sq_my + svq_my) : area * 0.0;
         double rhs = (double)fim[k] - (double)fip[k] + (double)fjm[k] - (double)fjp[k] + src;
-        if (MODE == RES_NR || MODE == RES_DUAL) {
+        if (MODE == RES_NR) {
             const double qk = v.q[k * N + c], qpk = v.qp[k * N + c];
             const double dqdt = first ? (qk - qpk) / dtl : (3.0 * qk - 4.0 * qpk + v.qpp[k * N + c]) / (2.0 * dtl);
             rhs = rhs - vol * dqdt;
@@ -347,49 +301,6 @@ __global__ void __launch_bounds__(NT) k_residual(View v) {
     const double cs = sqrt(gamm * pr / rho);
     const double unA = v.vnci[c] * u + v.vnci[N + c] * vv;
     const double unB = v.vncj[c] * u + v.vncj[N + c] * vv;
-    if (MODE == RES_DUAL) {
-        // set_ABpm of the preconditioned dual time (dual/2d/sch_dual.raw.f90:38-83):
-        // low-Mach reference velocity, preconditioned spectral radii, pseudo time
-        // step from cfl_tau, and the scalars of Gamma^-1, S, S^-1
-        const double mu = v.w[(D + 4) * N + c], dsa = v.dsci[c], dsb = v.dscj[c];
-        const double Vs = u * u + vv * vv;
-        const double Vv = mu / rho / fmin(dsa, dsb);
-        const double Ur = fmin(fmax(Vv, sqrt(Vs)), cs);
-        const double phi = 1.0 / (Ur * Ur) - 1.0 / (cs * cs);
-        const double alp = 0.5 * (1.0 - (Ur / cs) * (Ur / cs));
-        double ud = unA * (1.0 - alp), cd = sqrt(alp * alp * (unA * unA) + Ur * Ur);
-        const double nuA = fabs(ud) + cd;
-        ud = unB * (1.0 - alp);
-        cd = sqrt(alp * alp * (unB * unB) + Ur * Ur);
-        const double nuB = fabs(ud) + cd;
-        const long long cim = cidx(v.P, p, i - 1, j), cjm = cidx(v.P, p, i, j - 1);
-        const double uds = nuA * (v.dsi[c] + v.dsi[cim]) + nuB * (v.dsj[c] + v.dsj[cjm]);
-        const double dtau = v.cfl_tau * vol / fmax(uds, mu / rho);
-        const double al = 1.0 / (vol / dtau + dsa * nuA + dsb * nuB);
-        const double beta = 3.0 * vol / (2.0 * dtl) * al;
-        const double c2 = cs * cs;
-        const double s2 = -1.0 / (1.0 / phi + c2);
-        v.alpha[c] = al;
-        v.nuA[c] = nuA;
-        v.nuB[c] = nuB;
-        v.pre[c] = 1.0 + beta;
-        v.pre[N + c] = s2;
-        v.pre[2 * N + c] = -1.0 / (1.0 / phi + c2) / (1.0 / beta + 1.0);
-        v.pre[3 * N + c] = beta / ((1.0 + beta) / phi + c2);
-        // Dq += pre_sca(2) * (pre2 . Dq) * pre1 (time_dual_viscous.f90:29), pre1 =
-        // (Y, u, v, H), pre2 = (g1 Vs/2 + DHi, -g1 u, -g1 v, g1)
-        const double g1 = gamm - 1.0, H = v.w[(D + 2) * N + c];
-        double t = 0.0;
-        for (int k = 0; k < nY; ++k) t = t + (0.5 * g1 * Vs + v.DHi[k * N + c]) * v.Dq[k * N + c];
-        t = t + (-g1 * u) * v.Dq[nY * N + c];
-        t = t + (-g1 * vv) * v.Dq[(nY + 1) * N + c];
-        t = t + g1 * v.Dq[(nY + 2) * N + c];
-        for (int k = 0; k < nY; ++k) v.Dq[k * N + c] = v.Dq[k * N + c] + s2 * t * v.w[(4 + k) * N + c];
-        v.Dq[nY * N + c] = v.Dq[nY * N + c] + s2 * t * u;
-        v.Dq[(nY + 1) * N + c] = v.Dq[(nY + 1) * N + c] + s2 * t * vv;
-        v.Dq[(nY + 2) * N + c] = v.Dq[(nY + 2) * N + c] + s2 * t * H;
-        return;
-    }
     const double nuA = fabs(unA) + cs, nuB = fabs(unB) + cs;
     const double tmp = MODE == RES_NR ? 3.0 * vol / (2.0 * dtl) + v.dsci[c] * nuA + v.dscj[c] * nuB
                                       : vol / dtl + v.dsci[c] * nuA + v.dscj[c] * nuB;
@@ -417,12 +328,11 @@ static void launch_t(const View& v, cudaStream_t s) {
     k_residual<RT, MODE><<<grid, NT, smem, s>>>(v);
 }
 
-// need_coeffs: the caller's sweep reads alpha/nuA/nuB from the cell arrays,
-// which only this generic kernel writes.
+// need_coeffs: the caller's sweep reads alpha/nuA/nuB of plain LU-SGS / NR from the cell
+// arrays, which only this generic kernel writes.
 int launch_residual(const View& v, cudaStream_t s, int mode, bool need_coeffs) {
-    if (mode != RES_DUAL && mode != RES_PRECON && mode != RES_PRECON_LUSGS && !need_coeffs &&
-        launch_residual2(v, s, mode))
-        return 1;
+    const bool precond = mode == RES_DUAL || mode == RES_PRECON || mode == RES_PRECON_LUSGS;
+    if (!need_coeffs && (!precond || v.nY == 1) && launch_residual2(v, s, mode)) return 1;
     const bool mixed = v.precision == SCFD_PREC_MIXED;
     if (mode == RES_EULER) {
         if (mixed) launch_t<float, RES_EULER>(v, s); else launch_t<double, RES_EULER>(v, s);

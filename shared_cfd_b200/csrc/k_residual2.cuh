@@ -28,7 +28,7 @@
 #pragma once
 
 #include "div_pos.cuh"
-#include "scfd_internal.h"
+#include "precond.cuh"
 
 namespace scfd {
 
@@ -352,6 +352,16 @@ __global__ void __launch_bounds__(TL::NTH, sizeof(RT) == 4 ? TL::MINB : 0) k_res
     }
     const double vol = v.Vol[c];
     const bool first = v.sc->first_dual != 0;
+    if constexpr (MODE == RES_DUAL || MODE == RES_PRECON || MODE == RES_PRECON_LUSGS) {
+        double rhs[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            const double src = k == NY + 1 ? area * (sq_my + svq_my) : area * 0.0;
+            rhs[k] = flux_sum(k) + src;
+        }
+        precond_cell<MODE>(v, p, i, j, c, D, rhs, vol, dtl, first);
+        return;
+    }
     // all loads before the first store, so that they overlap
     double dq[D];
     if constexpr (MODE == RES_NR) {
@@ -409,8 +419,16 @@ inline void by_mode_rt(const View& v, cudaStream_t s, int mode) {
         by_tile<RT, NY, RES_EULER>(v, s);
     else if (mode == RES_LUSGS)
         by_tile<RT, NY, RES_LUSGS>(v, s);
-    else
+    else if (mode == RES_NR)
         by_tile<RT, NY, RES_NR>(v, s);
+    if constexpr (NY == 1) {  // the preconditioned schemes (launch_residual)
+        if (mode == RES_DUAL)
+            by_tile<RT, NY, RES_DUAL>(v, s);
+        else if (mode == RES_PRECON)
+            by_tile<RT, NY, RES_PRECON>(v, s);
+        else if (mode == RES_PRECON_LUSGS)
+            by_tile<RT, NY, RES_PRECON_LUSGS>(v, s);
+    }
 }
 
 // the launchers of one record precision (k_residual2_f32.cu, k_residual2_f64.cu);

@@ -425,9 +425,20 @@ void collect_events(scfd_ctx* c) {
 // generic one (the conditions of launch_residual and launch_residual2).
 bool fused_residual(const scfd_ctx* c) {
     const int sch = c->d.scheme;
-    if (sch == SCFD_SCHEME_DUAL || precon_scheme(sch)) return false;
     if (sch != SCFD_SCHEME_EULER && !c->use_sw3) return false;
-    return c->nY == 1 || c->nY == 8 || c->nY == 9;
+    return c->nY == 1 || (!preconditioned_scheme(sch) && (c->nY == 8 || c->nY == 9));
+}
+
+// the residual mode of a scheme
+int residual_mode(int scheme) {
+    switch (scheme) {
+        case SCFD_SCHEME_EULER: return RES_EULER;
+        case SCFD_SCHEME_LUSGS: return RES_LUSGS;
+        case SCFD_SCHEME_DUAL: return RES_DUAL;
+        case SCFD_SCHEME_PRECON: return RES_PRECON;
+        case SCFD_SCHEME_PRECON_LUSGS: return RES_PRECON_LUSGS;
+        default: return RES_NR;
+    }
 }
 
 // The kernels of one physical step, stage by stage; n counts the launches.
@@ -461,10 +472,8 @@ struct Seq {
         const long long qbytes = sizeof(double) * (long long)c->D * c->ncell;
         timed(c, SCFD_K_COPY, [&] { return (int)(cudaMemcpyAsync(dst, src, qbytes, cudaMemcpyDeviceToDevice, s) ? 0 : 0); });
     }
-    void residual(int mode) {
-        if (mode == RES_NR && c->d.scheme == SCFD_SCHEME_DUAL) mode = RES_DUAL;
-        if (mode == RES_NR && c->d.scheme == SCFD_SCHEME_PRECON) mode = RES_PRECON;
-        if (mode == RES_LUSGS && c->d.scheme == SCFD_SCHEME_PRECON_LUSGS) mode = RES_PRECON_LUSGS;
+    void residual() {
+        const int mode = residual_mode(c->d.scheme);
         const bool coeffs = mode != RES_EULER && !c->use_sw3;
         n += timed(c, SCFD_K_RESIDUAL, [&] { return launch_residual(v, s, mode, coeffs); });
     }
@@ -527,7 +536,7 @@ int enqueue_step(scfd_ctx* c) {
         for (int j = 1; j < c->d.num_internal_loop; ++j) {
             q.primitive(j == 1 ? PRO_QP | PRO_QPP : 0);
             q.bc();
-            q.residual(RES_NR);
+            q.residual();
             q.sweeps();
             q.update(j, q.partials(), q.nstrips());
         }
@@ -547,10 +556,8 @@ int enqueue_step(scfd_ctx* c) {
             if (c->d.dt_mode == SCFD_DT_GLOBAL) q.dtfinal();
         }
         q.bc();
-        if (c->d.scheme == SCFD_SCHEME_EULER) {
-            q.residual(RES_EULER);
-        } else {
-            q.residual(RES_LUSGS);
+        q.residual();
+        if (c->d.scheme != SCFD_SCHEME_EULER) {
             q.sweeps();
             q.update(1, q.partials(), q.nstrips());
         }
@@ -1185,10 +1192,8 @@ static int autotune(scfd_ctx* c) {
     char buf[512];
     std::string rep = "{\"enabled\": true";
     // residual: the fused kernel of the strip-record path (not the generic one)
-    const int mode = c->d.scheme == SCFD_SCHEME_EULER ? RES_EULER : c->d.scheme == SCFD_SCHEME_LUSGS ? RES_LUSGS : RES_NR;
-    const bool fused = c->d.scheme != SCFD_SCHEME_DUAL && !precon_scheme(c->d.scheme) &&
-                       (mode == RES_EULER || c->use_sw3) &&
-                       (c->nY == 1 || c->nY == 8 || c->nY == 9) && c->P.nact > 0;
+    const int mode = residual_mode(c->d.scheme);
+    const bool fused = fused_residual(c) && c->P.nact > 0;
     const char* force = std::getenv("SCFD_RES_TILE");  // pins the tile (index), e.g. for profiling
     int tx[8], ty[8];
     const int nt = residual2_tiles(tx, ty);
@@ -1414,7 +1419,7 @@ int scfd_dstep(scfd_ctx* c, int step, scfd_dreq* req, scfd_stats* stats) {
             case DS_AFTER_HALO_NR:
                 q.n += launch_halo_unpack(v, s, c->d_imp, c->nimp, c->d_halo);
                 q.bc();
-                q.residual(RES_NR);
+                q.residual();
                 q.sweeps();
                 q.n += launch_res_export(v, s, q.partials(), c->nsf == 0 ? 0 : q.nstrips(), c->d_red);
                 reduce(1, 2, DS_AFTER_RES);
@@ -1429,10 +1434,8 @@ int scfd_dstep(scfd_ctx* c, int step, scfd_dreq* req, scfd_stats* stats) {
             case DS_AFTER_HALO:
                 q.n += launch_halo_unpack(v, s, c->d_imp, c->nimp, c->d_halo);
                 q.bc();
-                if (c->d.scheme == SCFD_SCHEME_EULER) {
-                    q.residual(RES_EULER);
-                } else {
-                    q.residual(RES_LUSGS);
+                q.residual();
+                if (c->d.scheme != SCFD_SCHEME_EULER) {
                     q.sweeps();
                     q.update(1, q.partials(), q.nstrips());
                 }
