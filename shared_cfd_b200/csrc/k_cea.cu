@@ -32,6 +32,7 @@
 #include <string>
 #include <vector>
 
+#include "div_pos.cuh"
 #include "scfd_internal.h"
 
 namespace {
@@ -88,10 +89,24 @@ __device__ __forceinline__ int tsection(const double* thi, double tlo, int nsec,
     return nsec - 1;
 }
 
+// x / D for a small whole number D: the product with its reciprocal and Markstein's
+// remainder correction, without the division's out-of-line slow path
+template <int D>
+__device__ __forceinline__ double over(double x) {
+    constexpr double r = 1.0 / D;
+    const double q = x * r;
+    return fma(fma(-(double)D, q, x), r, q);
+}
+// x / a from y, a's reciprocal to within an ulp (as div_pos, of either sign)
+__device__ __forceinline__ double by_recip(double x, double a, double y) {
+    const double q = x * y;
+    return fma(fma(-a, q, x), y, q);
+}
+
 // calc_vThrt, calc_vTcpr, calc_vTmurt (func_chem.f90:63-148), in their
 // multiplication order
 __device__ __forceinline__ void v_hrt(double T, double logT, double* v) {
-    double tt = 1.0 / (T * T);
+    double tt = scfd::div_pos(1.0, T * T);
     v[0] = -tt;
     tt = tt * T;
     v[1] = tt * logT;
@@ -99,17 +114,17 @@ __device__ __forceinline__ void v_hrt(double T, double logT, double* v) {
     tt = tt * T;
     v[2] = tt;
     tt = tt * T;
-    v[3] = tt / 2.0;
+    v[3] = tt * 0.5;
     tt = tt * T;
-    v[4] = tt / 3.0;
+    v[4] = over<3>(tt);
     tt = tt * T;
-    v[5] = tt / 4.0;
+    v[5] = tt * 0.25;
     tt = tt * T;
-    v[6] = tt / 5.0;
+    v[6] = over<5>(tt);
     v[8] = 0.0;
 }
 __device__ __forceinline__ void v_cpr(double T, double* v) {
-    double tt = 1.0 / (T * T);
+    double tt = scfd::div_pos(1.0, T * T);
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
         v[k] = tt;
@@ -119,8 +134,8 @@ __device__ __forceinline__ void v_cpr(double T, double* v) {
     v[8] = 0.0;
 }
 __device__ __forceinline__ void v_murt(double T, double logT, double* v) {
-    double tt = 1.0 / (T * T);
-    v[0] = -tt / 2.0;
+    double tt = scfd::div_pos(1.0, T * T);
+    v[0] = -tt * 0.5;
     tt = tt * T;
     v[1] = tt * (1.0 + logT);
     v[7] = tt;
@@ -128,13 +143,13 @@ __device__ __forceinline__ void v_murt(double T, double logT, double* v) {
     v[2] = tt * (1.0 - logT);
     v[8] = -tt;
     tt = tt * T;
-    v[3] = -tt / 2.0;
+    v[3] = -tt * 0.5;
     tt = tt * T;
-    v[4] = -tt / 6.0;
+    v[4] = over<6>(-tt);
     tt = tt * T;
-    v[5] = -tt / 12.0;
+    v[5] = over<12>(-tt);
     tt = tt * T;
-    v[6] = -tt / 20.0;
+    v[6] = over<20>(-tt);
 }
 __device__ __forceinline__ double dot9(const double* c, const double* v) {
     double s = 0.0;
@@ -245,7 +260,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
         counter = 1;
         bool retried = false;
         for (;;) {
-            const double b0E = E / (RU * T);
+            const double b0E = scfd::div_pos(E, RU * T);
             double A[M][M], bd[M], vpi[M];
 #pragma unroll
             for (int i = 0; i < NE; ++i) {
@@ -303,6 +318,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
             // LU.f90: partial pivoting (first largest |A(i,k)|), singular when
             // the pivot is below 1e-30
             bool sing = false;
+            double rp[M];  // reciprocals of the pivots (of either sign, above 1e-30)
 #pragma unroll
             for (int k = 0; k < M; ++k) {
                 double p = fabs(A[k][k]);
@@ -331,7 +347,8 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
                     bd[k] = sw ? y : x;
                     bd[i] = sw ? x : y;
                 }
-                const double inv = 1.0 / A[k][k];
+                const double inv = scfd::div_pos(1.0, A[k][k]);
+                rp[k] = inv;
 #pragma unroll
                 for (int i = k + 1; i < M; ++i) A[i][k] = A[i][k] * inv;
 #pragma unroll
@@ -375,13 +392,13 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
 #pragma unroll
                 for (int j = 0; j < k; ++j) cc[k] = cc[k] - A[k][j] * cc[j];
             }
-            vpi[M - 1] = cc[M - 1] / A[M - 1][M - 1];
+            vpi[M - 1] = by_recip(cc[M - 1], A[M - 1][M - 1], rp[M - 1]);
 #pragma unroll
             for (int k = M - 2; k >= 0; --k) {
                 double x = cc[k];
 #pragma unroll
                 for (int j = k + 1; j < M; ++j) x = x - A[k][j] * vpi[j];
-                vpi[k] = x / A[k][k];
+                vpi[k] = by_recip(x, A[k][k], rp[k]);
             }
 #pragma unroll
             for (int r = 0; r < NE; ++r)
@@ -454,7 +471,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
     for (int j = 0; j < NS; ++j)
         if (j < ns) n_io[(int64_t)j * ncell + c] = n[j];
     if (out.iters) out.iters[c] = singular ? -1 : counter;
-    if (out.mwave) out.mwave[c] = 1e3 / sn;
+    if (out.mwave) out.mwave[c] = scfd::div_pos(1e3, sn);
 
     // kappa, vhi, DHi (sub_chem.f90:1596-1628)
     double vc[9];
@@ -463,7 +480,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
 #pragma unroll
     for (int i = 0; i < NS; ++i)
         if (i < ns && n[i] > tinyn) kap += n[i] * dot9(t.co[i][section<Tab, NSEC>(t, i, T)], vc);
-    kap = kap / (kap - sn);
+    kap = scfd::div_pos(kap, kap - sn);
     if (out.kappa) out.kappa[c] = kap;
     const double rt = RU * T;
     double vhe[NE], mwd[NE];
@@ -473,7 +490,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
     for (int i = 0; i < NS; ++i) {
         if (i >= ns) continue;
         const double dh = dot9(t.co[i][section<Tab, NSEC>(t, i, T)], vh);
-        if (out.vhi) out.vhi[(int64_t)i * ncell + c] = rt / t.mw[i] * dh * 1e3;
+        if (out.vhi) out.vhi[(int64_t)i * ncell + c] = scfd::div_pos(rt, t.mw[i]) * dh * 1e3;
         const double tmp2 = rt * n[i] * dh;
 #pragma unroll
         for (int j = 0; j < NE; ++j) {
@@ -487,7 +504,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
 #pragma unroll
         for (int i = 0; i < NE; ++i) {
             if (i >= ne) continue;
-            const double x = 1.0 / (Y0 * t.yfe[i] + Y1 * t.yoe[i] + 1e-300) *
+            const double x = scfd::div_pos(1.0, Y0 * t.yfe[i] + Y1 * t.yoe[i] + 1e-300) *
                              (kap * RU * mwd[i] * T - (kap - 1.0) * vhe[i]);
             d0 += t.yfe[i] * x;
             d1 += t.yoe[i] * x;
@@ -502,7 +519,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
     }
     if (out.mu) {
         // calc_vTmu (func_chem.f90:143-155) and the Wilke mixing rule
-        const double tt = 1.0 / (T * T);
+        const double tt = scfd::div_pos(1.0, T * T);
         const double vmu1 = tt * T, vmu2 = tt;
         // sqrt(muN_i / muN_j) as sqrt(muN_i) * rsqrt(muN_j): nt square roots
         // instead of nt^2 (a few ulp apart from the quotient's root)
@@ -537,7 +554,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
                 const double phi = 0.25 * (f * f) * t.wsq[i][j];
                 denom += nfit[j] * phi;
             }
-            mu += nfit[i] * (sq[i] * sq[i]) / denom;
+            mu += scfd::div_pos(nfit[i] * (sq[i] * sq[i]), denom);
         }
         out.mu[c] = mu * 1e-7;
     }
