@@ -30,6 +30,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "div_pos.cuh"
@@ -54,7 +55,7 @@ struct CeaTab {
     int tr2th[NS];
     double tlo[NS];              // Trange(1,1,j)
     double thi[NS][NSEC];        // Trange(2,l,j)
-    double co[NS][NSEC][9];
+    alignas(16) double co[NS][NSEC][10];  // 9 and a pad: rows of 16-byte vectors
     double mw[NS];
     double ac[NE][NS];
     double yac[NE][NS];
@@ -152,10 +153,15 @@ __device__ __forceinline__ void v_murt(double T, double logT, double* v) {
     v[6] = over<20>(-tt);
 }
 __device__ __forceinline__ double dot9(const double* c, const double* v) {
+    const double2* c2 = reinterpret_cast<const double2*>(c);
     double s = 0.0;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) s += c[k] * v[k];
-    return s;
+    for (int k = 0; k < 4; ++k) {
+        const double2 x = c2[k];
+        s += x.x * v[2 * k];
+        s += x.y * v[2 * k + 1];
+    }
+    return s + c[8] * v[8];
 }
 
 struct CellOut {
@@ -168,16 +174,37 @@ struct CellOut {
     int32_t* iters;
 };
 
+constexpr int kCeaThreads = 128;
+
+template <int NT>
+struct SmemVec {
+    double* p;
+    __device__ __forceinline__ explicit SmemVec(double* q) : p(q) {}
+    __device__ __forceinline__ double& operator[](int j) const { return p[j * NT]; }
+};
+template <int NS>
+struct RegVec {
+    double a[NS];
+    __device__ __forceinline__ explicit RegVec(double*) {}
+    __device__ __forceinline__ double& operator[](int j) { return a[j]; }
+    __device__ __forceinline__ const double& operator[](int j) const { return a[j]; }
+};
+
 // EXACT: the species set has exactly NS species and NE elements, so that the
 // counts are compile-time constants and no register holds an unused slot.
-template <int NS, int NE, int NSEC, bool EXACT, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* __restrict__ gtab, int64_t ncell,
+// SMEM: the species vectors lie in shared memory, one column per thread, and the
+// species loops are rolled: a ninth of the code (in registers, fully unrolled, 18 k
+// instructions a warp, a tenth of the time waiting for instructions, 40 % for the FP64
+// chains of 11.5 resident warps) and 80 registers less, so 16 to 20 warps are resident.
+// Same arithmetic in the same order.
+template <int NS, int NE, int NSEC, bool EXACT, int MINB, bool SMEM>
+__global__ void __launch_bounds__(kCeaThreads, MINB) k_cea(const CeaTab<NS, NE, NSEC>* __restrict__ gtab, int64_t ncell,
                                              const double* __restrict__ rho_in, const double* __restrict__ Y_in,
                                              const double* __restrict__ E_in, double* __restrict__ T_io,
                                              double* __restrict__ n_io, CellOut out,
                                              unsigned long long* __restrict__ fails) {
     using Tab = CeaTab<NS, NE, NSEC>;
-    extern __shared__ double smem_tab[];
+    extern __shared__ __align__(16) double smem_tab[];
     {
         const double* src = reinterpret_cast<const double*>(gtab);
         for (int k = threadIdx.x; k < (int)(sizeof(Tab) / sizeof(double)); k += blockDim.x) smem_tab[k] = src[k];
@@ -191,8 +218,12 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
 
     const double rho = rho_in[c], Y0 = Y_in[c], Y1 = Y_in[ncell + c], E = E_in[c];
     double T = T_io[c];
-    double n[NS], logn[NS], vert[NS], dl[NS];
-#pragma unroll
+    // the species vectors: in shared memory, one column per thread, or in registers
+    using Vec = typename std::conditional<SMEM, SmemVec<kCeaThreads>, RegVec<NS>>::type;
+    double* const col = smem_tab + sizeof(Tab) / sizeof(double) + threadIdx.x;
+    Vec n(col), logn(col + NS * kCeaThreads), vert(col + 2 * NS * kCeaThreads), dl(col + 3 * NS * kCeaThreads);
+    constexpr int UN = SMEM ? 1 : NS;  // species loops: rolled where indices may vary
+#pragma unroll UN
     for (int j = 0; j < NS; ++j) n[j] = j < ns ? n_io[(int64_t)j * ncell + c] : 0.0;
 
     const double logrhoRu = log(rho * RU / PST);
@@ -210,7 +241,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
         if (i < ne && b0[i] > b0max) b0max = b0[i];
     const int mode = Y0 < Y_EPS ? 1 : (Y1 < Y_EPS ? 2 : 0);
     if (mode) {
-#pragma unroll
+#pragma unroll UN
         for (int j = 0; j < NS; ++j)
             if (j < ns) n[j] = n[j] * (mode == 1 ? t.masko[j] : t.maskf[j]);
 #pragma unroll
@@ -220,7 +251,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
         }
     }
     double sn = 0.0;
-#pragma unroll
+#pragma unroll UN
     for (int j = 0; j < NS; ++j)
         if (j < ns) sn += n[j];
     const double tinyn = TSIZE * sn;
@@ -234,7 +265,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
     double b[NE], bE = 0.0;
 #pragma unroll
     for (int i = 0; i < NE; ++i) b[i] = 0.0;
-#pragma unroll
+#pragma unroll UN
     for (int j = 0; j < NS; ++j) {
         vert[j] = 0.0;
         logn[j] = logtinyn;
@@ -276,7 +307,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
             v_murt(T, logT, vm);
             v_cpr(T, vc);
             double aEE = 0.0;
-#pragma unroll
+#pragma unroll UN
             for (int k = 0; k < NS; ++k) {
                 if (k >= ns) continue;
                 const int s = section<Tab, NSEC>(t, k, T);
@@ -365,7 +396,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
                 }
                 retried = true;
                 bE = 0.0;
-#pragma unroll
+#pragma unroll UN
                 for (int j = 0; j < NS; ++j) {
                     if (j >= ns) continue;
                     n[j] = n[j] + INITIAL_EPS;
@@ -380,7 +411,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
                     }
                 }
                 sn = 0.0;
-#pragma unroll
+#pragma unroll UN
                 for (int j = 0; j < NS; ++j)
                     if (j < ns) sn += n[j];
                 continue;
@@ -405,7 +436,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
                 if (r < ne && keep[r] == 0.0) vpi[r] = -1e300;
 
             const double dlogT = vpi[NE];
-#pragma unroll
+#pragma unroll UN
             for (int j = 0; j < NS; ++j) {
                 if (j >= ns) continue;
                 double s = 0.0;
@@ -416,7 +447,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
             }
             double lambda1 = 0.0, lambda2 = 1e300;
             const double logsn = log(sn);
-#pragma unroll
+#pragma unroll UN
             for (int j = 0; j < NS; ++j) {
                 if (j >= ns) continue;
                 if (logn[j] - logsn > -18.420681)
@@ -432,7 +463,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
             bE = 0.0;
             double dnmax = 0.0;
             v_hrt(T, logT, vh);
-#pragma unroll
+#pragma unroll UN
             for (int j = 0; j < NS; ++j) {
                 if (j >= ns) continue;
                 n[j] = n[j] * exp(om * dl[j]);
@@ -449,7 +480,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
                 }
             }
             sn = 0.0;
-#pragma unroll
+#pragma unroll UN
             for (int j = 0; j < NS; ++j)
                 if (j < ns) sn += n[j];
             flag = true;
@@ -467,7 +498,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
     else if (counter > MAX_ITER) atomicAdd(&fails[0], 1ull);
 
     T_io[c] = T;
-#pragma unroll
+#pragma unroll UN
     for (int j = 0; j < NS; ++j)
         if (j < ns) n_io[(int64_t)j * ncell + c] = n[j];
     if (out.iters) out.iters[c] = singular ? -1 : counter;
@@ -477,7 +508,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
     double vc[9];
     v_cpr(T, vc);
     double kap = 0.0;
-#pragma unroll
+#pragma unroll UN
     for (int i = 0; i < NS; ++i)
         if (i < ns && n[i] > tinyn) kap += n[i] * dot9(t.co[i][section<Tab, NSEC>(t, i, T)], vc);
     kap = scfd::div_pos(kap, kap - sn);
@@ -486,7 +517,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
     double vhe[NE], mwd[NE];
 #pragma unroll
     for (int i = 0; i < NE; ++i) vhe[i] = mwd[i] = 0.0;
-#pragma unroll
+#pragma unroll UN
     for (int i = 0; i < NS; ++i) {
         if (i >= ns) continue;
         const double dh = dot9(t.co[i][section<Tab, NSEC>(t, i, T)], vh);
@@ -513,7 +544,7 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
         out.DHi[ncell + c] = d1;
     }
     if (out.Yv) {
-#pragma unroll
+#pragma unroll UN
         for (int i = 0; i < NS; ++i)
             if (i < ns) out.Yv[(int64_t)i * ncell + c] = n[i] * t.mw[i] * 1e-3;
     }
@@ -523,8 +554,9 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
         const double vmu1 = tt * T, vmu2 = tt;
         // sqrt(muN_i / muN_j) as sqrt(muN_i) * rsqrt(muN_j): nt square roots
         // instead of nt^2 (a few ulp apart from the quotient's root)
-        double sq[NS], rs[NS];
-#pragma unroll
+        Vec& sq = logn;  // reused: ln n and its step are done with
+        Vec& rs = dl;
+#pragma unroll UN
         for (int i = 0; i < NS; ++i) {
             sq[i] = rs[i] = 0.0;
             if (i >= nt) continue;
@@ -534,20 +566,24 @@ __global__ void __launch_bounds__(128, MINB) k_cea(const CeaTab<NS, NE, NSEC>* _
             sq[i] = sqrt(muN);
             rs[i] = rsqrt(muN);
         }
-        double nfit[NS];  // n(tr2th(i))
-#pragma unroll
+        Vec& nfit = vert;  // n(tr2th(i))
+#pragma unroll UN
         for (int i = 0; i < NS; ++i) {
             nfit[i] = 0.0;
-#pragma unroll
-            for (int k = 0; k < NS; ++k)
-                if (i < nt && k == t.tr2th[i]) nfit[i] = n[k];
+            if constexpr (SMEM) {
+                if (i < nt) nfit[i] = n[t.tr2th[i]];
+            } else {
+#pragma unroll UN
+                for (int k = 0; k < NS; ++k)
+                    if (i < nt && k == t.tr2th[i]) nfit[i] = n[k];
+            }
         }
         double mu = 0.0;
-#pragma unroll
+#pragma unroll UN
         for (int i = 0; i < NS; ++i) {
             if (i >= nt) continue;
             double denom = 0.0;
-#pragma unroll
+#pragma unroll UN
             for (int j = 0; j < NS; ++j) {
                 if (j >= nt) continue;
                 const double f = 1.0 + sq[i] * rs[j] * t.wmw[i][j];
@@ -1005,19 +1041,32 @@ namespace {
 int cea_launch(scfd_cea* h, int64_t ncell, const double* rho, const double* Y, const double* e, double* T,
                double* n, const CellOut& out, cudaStream_t st) {
     if (ncell == 0) return 0;
-    const int threads = 128;
+    const int threads = kCeaThreads;
     const int64_t blocks = (ncell + threads - 1) / threads;
     if (blocks > 0x7fffffff) return SCFD_E_ARG;
-    // three resident blocks of 128 threads (168 registers) measured faster
-    // than two (no spills) and than four (more spills) on B200
-    if (h->kind == KIND_9_3)
-        k_cea<9, 3, 3, true, 3><<<(unsigned)blocks, threads, sizeof(TabH2Air), st>>>(
-            (const TabH2Air*)h->d_tab, ncell, rho, Y, e, T, n, out, h->d_fail);
-    else if (h->kind == KIND_SMALL)
-        k_cea<12, 4, 3, false, 3><<<(unsigned)blocks, threads, sizeof(TabSmall), st>>>(
+    constexpr size_t kCeaExactSmem = sizeof(TabH2Air) + sizeof(double) * 4 * 9 * kCeaThreads;
+    if (h->kind == KIND_9_3) {
+        // Register vectors (3 blocks per SM) while one wave holds the batch: a cell's own
+        // latency counts there (4099 cells 58 us, 40 000 cells 70 us, against 68 and 77).
+        // Above that the shared-memory vectors, whose small code and more resident warps
+        // win (2^17 cells 162 us against 192): 4 blocks per SM without spills, and 5 for four
+        // waves and more (2^20 cells 1093 us against 1133, and 1285 in registers).
+        int dev = 0, nsm = 148;
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        if (blocks <= 3ll * nsm)
+            k_cea<9, 3, 3, true, 3, false><<<(unsigned)blocks, threads, sizeof(TabH2Air), st>>>(
+                (const TabH2Air*)h->d_tab, ncell, rho, Y, e, T, n, out, h->d_fail);
+        else if (blocks < 20ll * nsm)
+            k_cea<9, 3, 3, true, 4, true><<<(unsigned)blocks, threads, kCeaExactSmem, st>>>(
+                (const TabH2Air*)h->d_tab, ncell, rho, Y, e, T, n, out, h->d_fail);
+        else
+            k_cea<9, 3, 3, true, 5, true><<<(unsigned)blocks, threads, kCeaExactSmem, st>>>(
+                (const TabH2Air*)h->d_tab, ncell, rho, Y, e, T, n, out, h->d_fail);
+    } else if (h->kind == KIND_SMALL)
+        k_cea<12, 4, 3, false, 3, false><<<(unsigned)blocks, threads, sizeof(TabSmall), st>>>(
             (const TabSmall*)h->d_tab, ncell, rho, Y, e, T, n, out, h->d_fail);
     else
-        k_cea<SCFD_CEA_MAX_SPECIES, SCFD_CEA_MAX_ELEMENTS, SCFD_CEA_MAX_SECTIONS, false, 1>
+        k_cea<SCFD_CEA_MAX_SPECIES, SCFD_CEA_MAX_ELEMENTS, SCFD_CEA_MAX_SECTIONS, false, 1, false>
             <<<(unsigned)blocks, threads, sizeof(TabBig), st>>>((const TabBig*)h->d_tab, ncell, rho, Y, e, T, n,
                                                                  out, h->d_fail);
     return cudaGetLastError() == cudaSuccess ? 0 : SCFD_E_CUDA;

@@ -209,3 +209,17 @@ def test_hp_stream_states_match(gpu, orc):
             x, y = getattr(a, s), getattr(b, s)
             for k in ("rho", "p", "T", "e", "h", "mw", "kappa", "mu"):
                 assert getattr(x, k) == pytest.approx(getattr(y, k), rel=1e-10), (s, k)
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 3 * 148 * 128 + 1, 20 * 148 * 128 + 77])
+def test_gpu_batch_sizes_take_the_same_values(gpu, n):
+    """The launch shape of the 9-species set follows the batch size (registers, shared
+    memory, more blocks): the same cells give the same bits in every one."""
+    d = cea.h2_air_data()
+    with cea.Cea(d, lib=gpu) as g:
+        rho, Y, e, T = cea.random_states(g.info(), 20 * 148 * 128 + 77, seed=5)
+        few = g.solve(rho[-64:], Y[:, -64:], e[-64:], T[-64:], g.initial_n(64))
+        got = g.solve(rho[-n:], Y[:, -n:], e[-n:], T[-n:], g.initial_n(n))
+        m = min(n, 64)
+        for k in ("T", "n", "MWave", "kappa", "mu", "Yv", "vhi", "DHi", "iters"):
+            np.testing.assert_array_equal(got[k][..., -m:], few[k][..., -m:], err_msg=k)
