@@ -1046,14 +1046,18 @@ int cea_launch(scfd_cea* h, int64_t ncell, const double* rho, const double* Y, c
     if (blocks > 0x7fffffff) return SCFD_E_ARG;
     constexpr size_t kCeaExactSmem = sizeof(TabH2Air) + sizeof(double) * 4 * 9 * kCeaThreads;
     if (h->kind == KIND_9_3) {
-        // Register vectors (3 blocks per SM) while one wave holds the batch: a cell's own
-        // latency counts there (4099 cells 58 us, 40 000 cells 70 us, against 68 and 77).
+        // Register vectors while one wave holds the batch: a cell's own latency counts there
+        // (4099 cells 54 us with the 255 registers that 2 blocks per SM leave, 58 with
+        // 3 blocks; 40 000 cells 70 us with 3; shared-memory vectors 68 and 77).
         // Above that the shared-memory vectors, whose small code and more resident warps
         // win (2^17 cells 162 us against 192): 4 blocks per SM without spills, and 5 for four
         // waves and more (2^20 cells 1093 us against 1133, and 1285 in registers).
         int dev = 0, nsm = 148;
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        if (blocks <= 3ll * nsm)
+        if (blocks <= 2ll * nsm)
+            k_cea<9, 3, 3, true, 2, false><<<(unsigned)blocks, threads, sizeof(TabH2Air), st>>>(
+                (const TabH2Air*)h->d_tab, ncell, rho, Y, e, T, n, out, h->d_fail);
+        else if (blocks <= 3ll * nsm)
             k_cea<9, 3, 3, true, 3, false><<<(unsigned)blocks, threads, sizeof(TabH2Air), st>>>(
                 (const TabH2Air*)h->d_tab, ncell, rho, Y, e, T, n, out, h->d_fail);
         else if (blocks < 20ll * nsm)

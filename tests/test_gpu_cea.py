@@ -211,7 +211,7 @@ def test_hp_stream_states_match(gpu, orc):
                 assert getattr(x, k) == pytest.approx(getattr(y, k), rel=1e-10), (s, k)
 
 
-@pytest.mark.parametrize("n", [1, 127, 129, 3 * 148 * 128 + 1, 20 * 148 * 128 + 77])
+@pytest.mark.parametrize("n", [1, 129, 2 * 148 * 128 + 1, 3 * 148 * 128 + 1, 20 * 148 * 128 + 77])
 def test_gpu_batch_sizes_take_the_same_values(gpu, n):
     """The launch shape of the 9-species set follows the batch size (registers, shared
     memory, more blocks): the same cells give the same bits in every one."""
