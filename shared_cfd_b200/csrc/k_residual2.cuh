@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(TL::NTH, sizeof(RT) == 4 ? TL::MINB : 0) k_res
 #pragma unroll
         for (int m = 0; m < W; ++m) S.w[m * HS + e] = RT(r[m]);
         const RT rr = RT(r[0]);
-        S.T[e] = rr != RT(0) ? RT(r[3]) / rr / RT(r[D + 3]) : RT(0);
+        if (v.viscous) S.T[e] = rr != RT(0) ? RT(r[3]) / rr / RT(r[D + 3]) : RT(0);
         if constexpr (NVH > 0) {
 #pragma unroll
             for (int m = 0; m < NVH; ++m) r[m] = in ? __ldg(v.vhi + m * N + c) : 0.0;

@@ -128,9 +128,22 @@ __device__ __forceinline__ void prologue(const View& v, int flags, bool in, int 
     const long long N = v.ncell;
     const long long c = in ? cidx(v.P, p, i, j) : 0;
     if (in && (flags & PRO_QP)) {
-        for (int k = 0; k < v.D; ++k) {
-            if (flags & PRO_QPP) v.qpp[k * N + c] = v.qp[k * N + c];
-            v.qp[k * N + c] = v.q[k * N + c];
+        // in batches, whose loads overlap
+        constexpr int NB = 6;
+        for (int k0 = 0; k0 < v.D; k0 += NB) {
+            double a[NB], b[NB];
+#pragma unroll
+            for (int e = 0; e < NB; ++e)
+                if (k0 + e < v.D) {
+                    a[e] = v.q[(k0 + e) * N + c];
+                    if (flags & PRO_QPP) b[e] = v.qp[(k0 + e) * N + c];
+                }
+#pragma unroll
+            for (int e = 0; e < NB; ++e)
+                if (k0 + e < v.D) {
+                    if (flags & PRO_QPP) v.qpp[(k0 + e) * N + c] = b[e];
+                    v.qp[(k0 + e) * N + c] = a[e];
+                }
         }
     }
     if (flags & PRO_DT) {
@@ -407,6 +420,77 @@ __global__ void __launch_bounds__(256) k_thermo(View v, int flags) {
     if (PRO) prologue(v, flags, in, p, i, j);
 }
 
+// k_thermo for the ideal gas (one species), straight through: every load first, the
+// prologue from registers.  The generic form read back what it had just written (sqrt of
+// gamma p / rho, q for the copies) and waited for each load of its species loops: 6.8 us
+// for 1600 cells and 10.4 us for 197 k with the prologue.  Same arithmetic.
+template <bool PRO>
+__global__ void __launch_bounds__(256) k_thermo_ideal(View v, int flags) {
+    const int p = v.P.act[blockIdx.y];
+    const int ni = v.P.ni[p], nj = v.P.nj[p];
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = idx < ni * nj;
+    const int i = idx % ni + 1, j = idx / ni + 1;
+    const long long N = v.ncell;
+    double dtc = 1e300;
+    if (in) {
+        const long long c = cidx(v.P, p, i, j);
+        constexpr int D = 4, ig = D + 1, iht = D + 2, iR = D + 3, imu = D + 4;
+        double q[D], qp[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k) q[k] = v.q[k * N + c];
+        if (PRO && (flags & PRO_QPP)) {
+#pragma unroll
+            for (int k = 0; k < D; ++k) qp[k] = v.qp[k * N + c];
+        }
+        const bool dt = PRO && (flags & PRO_DT) && v.dt_mode != SCFD_DT_FIXED;
+        const DtMetrics m(v, p, i, dt ? j : 1);
+        double* w = v.w;
+        const double rho = 0.0 + q[0];
+        const double tmp = 1.0 / rho;
+        const double u = q[1] * tmp, vv = q[2] * tmp;
+        const double qE = q[3];
+        const double ei = qE / rho - 0.5 * (u * u + vv * vv);
+        const double kg = v.kappa, Rg = v.rgas;
+        const double T = ei * (kg - 1.0) / Rg;
+        const double pr = rho * Rg * T;
+        double mu;
+        if (v.mu_model == SCFD_MU_SUTHERLAND)
+            mu = v.suth_mu0 * pow(T / v.suth_t0, 1.5) * (v.suth_t0 + v.suth_s) / (T + v.suth_s);
+        else
+            mu = rho * v.nu_gas;
+        if (dt) dtc = cell_dt(v, m, rho, u, vv, pr, kg, mu);
+        w[c] = rho;
+        w[N + c] = u;
+        w[2 * N + c] = vv;
+        w[3 * N + c] = pr;
+        w[4 * N + c] = q[0] * tmp;
+        w[ig * N + c] = kg;
+        w[iht * N + c] = (qE + pr) / rho;
+        w[iR * N + c] = Rg;
+        w[imu * N + c] = mu;
+        v.DHi[c] = 0.0;
+        v.vhi[c] = kg / (kg - 1.0) * Rg * T;
+        if (dt) v.dt_mat[c] = dtc;
+        if (PRO && (flags & PRO_QP)) {
+#pragma unroll
+            for (int k = 0; k < D; ++k) {
+                if (flags & PRO_QPP) v.qpp[k * N + c] = qp[k];
+                v.qp[k * N + c] = q[k];
+            }
+        }
+    }
+    if (PRO && (flags & PRO_DT)) {
+        if (v.dt_mode == SCFD_DT_FIXED) {
+            if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) dt_final(v);
+        } else if (v.dt_mode == SCFD_DT_GLOBAL) {
+            for (int o = 16; o > 0; o >>= 1) dtc = fmin(dtc, __shfl_xor_sync(0xffffffffu, dtc, o));
+            if ((threadIdx.x & 31) == 0 && dtc < 1e300)
+                atomicMin(&v.sc->dtmin_bits, (unsigned long long)__double_as_longlong(dtc));
+        }
+    }
+}
+
 int launch_thermo(const View& v, cudaStream_t s, int cells_per_plane_max, int prologue) {
     if (v.P.nact == 0) return 0;
     const int bs = v.thermo_block == 64 || v.thermo_block == 256 ? v.thermo_block : 128;
@@ -415,6 +499,9 @@ int launch_thermo(const View& v, cudaStream_t s, int cells_per_plane_max, int pr
     if (v.thermo != SCFD_THERMO_IDEAL && v.chem.ns == 9 && v.nY == 9 && v.chem.nt <= 9) {
         if (prologue) k_thermo_fixed<9, true><<<grid, bs, 0, s>>>(v, prologue);
         else k_thermo_fixed<9, false><<<grid, bs, 0, s>>>(v, 0);
+    } else if (v.thermo == SCFD_THERMO_IDEAL && v.nY == 1) {
+        if (prologue) k_thermo_ideal<true><<<grid, bs, 0, s>>>(v, prologue);
+        else k_thermo_ideal<false><<<grid, bs, 0, s>>>(v, 0);
     } else {
         if (prologue) k_thermo<true><<<grid, bs, 0, s>>>(v, prologue);
         else k_thermo<false><<<grid, bs, 0, s>>>(v, 0);
