@@ -73,8 +73,8 @@ struct scfd_ctx {
     // the whole physical step as one CUDA graph (captured at the second step)
     bool use_graph = true;
     int eager_steps = 0;
-    cudaGraphExec_t graph = nullptr;
-    long long graph_launches = 0;
+    cudaGraphExec_t graph = nullptr, graph_n = nullptr;  // one step; kGraphSteps steps
+    long long graph_launches = 0, graph_n_launches = 0;
     std::vector<cudaEvent_t> ev_pool;
     size_t ev_used = 0;
     std::vector<std::pair<int, size_t>> ev_marks;  // kind, index of the start event
@@ -649,6 +649,7 @@ int scfd_destroy(scfd_ctx* c) {
                     (void*)c->adj.ocells, (void*)c->adj.owt})
         if (b) cudaFree(b);
     if (c->graph) cudaGraphExecDestroy(c->graph);
+    if (c->graph_n) cudaGraphExecDestroy(c->graph_n);
     for (int b = 0; b < 2; ++b) {
         if (c->h_ring[b]) cudaFreeHost(c->h_ring[b]);
         if (c->ring_ev[b]) cudaEventDestroy(c->ring_ev[b]);
@@ -1258,6 +1259,36 @@ static int autotune(scfd_ctx* c) {
 // device pointers and host constants of the context only: dt, time and status
 // live on the device.  Profiled steps run eagerly (their events are recorded
 // between the kernels).
+namespace {
+// captures n steps; launches: how many kernels one replay runs
+int capture_steps(scfd_ctx* c, int n, cudaGraphExec_t* out, long long* launches) {
+    const long long before = c->launches;
+    cudaGraph_t g = nullptr;
+    CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+    int st = 0;
+    for (int k = 0; k < n && !st; ++k) st = enqueue_step(c);
+    const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+    *launches = c->launches - before;
+    c->launches = before;
+    if (st) {
+        if (g) cudaGraphDestroy(g);
+        return st;
+    }
+    if (e != cudaSuccess) return c->fail(SCFD_E_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+    const cudaError_t ei = cudaGraphInstantiate(out, g, 0);
+    cudaGraphDestroy(g);
+    if (ei != cudaSuccess) {
+        *out = nullptr;
+        return c->fail(SCFD_E_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ei));
+    }
+    return 0;
+}
+
+// Steps per replay of the long graph: the steps without an inner loop have 4 to 7 short
+// kernels, so that the gap between two graphs counts (Sod 15.0 -> 13.6 us a step).
+constexpr int kGraphSteps = 8;
+}  // namespace
+
 int step_once(scfd_ctx* c) {
     if (!c->tuned) {
         const int st = autotune(c);
@@ -1268,27 +1299,34 @@ int step_once(scfd_ctx* c) {
         return enqueue_step(c);
     }
     if (!c->graph) {
-        const long long before = c->launches;
-        cudaGraph_t g = nullptr;
-        CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        const int st = enqueue_step(c);
-        const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
-        if (st) {
-            if (g) cudaGraphDestroy(g);
-            return st;
-        }
-        if (e != cudaSuccess) return c->fail(SCFD_E_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-        const cudaError_t ei = cudaGraphInstantiate(&c->graph, g, 0);
-        cudaGraphDestroy(g);
-        if (ei != cudaSuccess) {
-            c->graph = nullptr;
-            return c->fail(SCFD_E_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ei));
-        }
-        c->graph_launches = c->launches - before;
-        c->launches = before;
+        const int st = capture_steps(c, 1, &c->graph, &c->graph_launches);
+        if (st) return st;
     }
     CK(cudaGraphLaunch(c->graph, c->stream));
     c->launches += c->graph_launches;
+    return 0;
+}
+
+// n steps, several to a graph where that pays
+int steps(scfd_ctx* c, int n) {
+    // a long graph is built for a run that replays it a few times
+    const bool many = (c->graph_n || n >= 4 * kGraphSteps) && !dual_time_scheme(c->d.scheme) && !c->profiling;
+    while (n > 0) {
+        if (many && c->graph && n >= kGraphSteps) {
+            if (!c->graph_n) {
+                const int st = capture_steps(c, kGraphSteps, &c->graph_n, &c->graph_n_launches);
+                if (st) return st;
+            }
+            CK(cudaGraphLaunch(c->graph_n, c->stream));
+            c->launches += c->graph_n_launches;
+            n -= kGraphSteps;
+            continue;
+        }
+        const int st = step_once(c);
+        if (st) return st;
+        --n;
+        if (c->profiling && c->ev_used > 4096) collect_events(c);
+    }
     return 0;
 }
 
@@ -1314,10 +1352,7 @@ int scfd_run(scfd_ctx* c, int step, int nsteps, scfd_stats* stats) {
     if (st) return st;
     const long long att0 = c->h_sc->chem_attempts, fb0 = c->h_sc->chem_fallback;
     c->launches = 0;
-    for (int n = 0; n < nsteps; ++n) {
-        if ((st = step_once(c))) return st;
-        if (c->profiling && c->ev_used > 4096) collect_events(c);
-    }
+    if ((st = steps(c, nsteps))) return st;
     if ((st = sync_scalars(c))) return st;
     collect_events(c);
     // the chemistry counts of the last step (a run of no step reports none)
@@ -1514,7 +1549,16 @@ struct AdjRun {
     }
     // q^a in the context -> q^b; adds the objective of states formed for the first time
     int advance(int a, int b) {
-        for (int k = a; k < b; ++k) {
+        // steps whose objective is not wanted (or known already) go several to a graph
+        int plain = a;
+        while (plain < b && (plain + 1 <= visited || !in_window(plain + 1))) ++plain;
+        if (plain > a) {
+            const int st = steps(c, plain - a);
+            if (st) return st;
+            fwd += plain - a;
+            visited = std::max(visited, plain);
+        }
+        for (int k = plain; k < b; ++k) {
             int st = step_once(c);
             if (st) return st;
             ++fwd;
