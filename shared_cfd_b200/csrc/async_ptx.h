@@ -77,33 +77,11 @@ __device__ __forceinline__ bool mbar_test_wait(unsigned long long* bar, unsigned
         : "memory");
     return ok != 0;
 }
-// try_wait with acquire at cluster scope: for phases completed by another CTA
-// of the cluster (st.async complete_tx, remote arrive)
-__device__ __forceinline__ bool mbar_try_wait_cluster(unsigned long long* bar, unsigned phase) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(phase)
-        : "memory");
-    return ok != 0;
-}
 
 // ---- thread-block clusters: rank, distributed shared memory -------------
 __device__ __forceinline__ unsigned cluster_rank() {
     unsigned r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned cluster_id_x() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned cluster_nclusters_x() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%nclusterid.x;" : "=r"(r));
     return r;
 }
 // all threads of all CTAs of the cluster (release / acquire at cluster scope)
@@ -116,23 +94,6 @@ __device__ __forceinline__ unsigned mapa(const void* p, unsigned rank) {
     unsigned r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
     return r;
-}
-// 16-byte store into another CTA's shared memory that completes 16 bytes of
-// transaction count on an mbarrier of that CTA
-__device__ __forceinline__ void st_async16(unsigned raddr, float4 v, unsigned rbar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
-                     raddr),
-                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(rbar)
-                 : "memory");
-}
-__device__ __forceinline__ void st_async16(unsigned raddr, double2 v, unsigned rbar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(raddr),
-                 "d"(v.x), "d"(v.y), "r"(rbar)
-                 : "memory");
-}
-// arrive (release, cluster scope) on an mbarrier given by its shared::cluster address
-__device__ __forceinline__ void mbar_arrive_cluster(unsigned rbar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(rbar) : "memory");
 }
 // the same without release semantics (no fence): for a consumer telling a
 // producer that a buffer may be refilled, where the consumer's reads of it
@@ -153,21 +114,7 @@ __device__ __forceinline__ void bulk_s2dsmem(unsigned rdst, const void* src, uns
                  "r"(smem_u32(src)), "r"(bytes), "r"(rbar)
                  : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
 
-// ---- bulk stores shared -> global and proxy fences ------------------------
-__device__ __forceinline__ void tma_bulk_s2g(void* gdst, const void* src, unsigned bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst), "r"(smem_u32(src)),
-                 "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// every committed bulk store has finished reading shared memory
-__device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// every committed bulk store has completed its global writes
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // generic-proxy shared-memory writes become visible to later bulk copies
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -175,11 +122,6 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 // generic-proxy global accesses are ordered with later bulk copies
 __device__ __forceinline__ void fence_proxy_async_global() {
     asm volatile("fence.proxy.async.global;" ::: "memory");
-}
-__device__ __forceinline__ int ld_relaxed_gpu(const int* p) {
-    int v;
-    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
 }
 
 }  // namespace ptx

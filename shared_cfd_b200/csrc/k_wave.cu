@@ -22,10 +22,11 @@
 // global memory (nothing waits for them), and record loads, the release of
 // consumed hand-off chunks and the hand-off itself have warps of their own.
 // Measured (B200, per launch, forward / backward): 786 k cells of 9 species FP64
-// 281 / 272 us, FP32 212 / 208 us, against 426 / 414 and 289 / 288 us for 32-row
-// strips with one lane per cell; 256 x 128 cells of one species FP64 74 / 72 us
-// against 103 / 101 us.  A step takes 195 (FP64) and 141 ns (FP32) at 9 species,
-// 138 and 100 ns at one, with or without hand-off (one lane per cell: 398, 255, 248, 180 ns).
+// 269 / 254 us, FP32 200 / 197 us, against 426 / 414 and 289 / 288 us for 32-row
+// strips with one lane per cell; 256 x 128 cells of one species FP64 70 / 68 us
+// against 103 / 101 us.  A step takes 190-196 (forward) and 185 ns (backward) FP64 and
+// 140 ns FP32 at 9 species, 135 and 98 ns at one (one lane per cell: 398, 255, 248 and
+// 180 ns), of which the hand-off is about 10.
 //
 // A task is 256 consecutive rows of one plane at most, run by one thread-block
 // cluster of 16 CTAs with two strips each.  A strip's top row is staged in its

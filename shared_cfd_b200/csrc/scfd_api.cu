@@ -820,7 +820,7 @@ int scfd_commit(scfd_ctx* c) {
     const ChemTables tabs = c->have_chem ? ChemTables(c->chem) : ChemTables();
     const int nrec = 64 * c->np;
     // strip records for the cluster-wavefront sweeps
-    // the dual and precon schemes take the generic residual and sweeps
+    // (the preconditioned schemes have them for one species)
     const bool dual = c->d.scheme == SCFD_SCHEME_DUAL || precon_scheme(c->d.scheme);
     const WaveSizes wz = impl ? wave_sizes(nY, mixed, dual) : WaveSizes{0, 0, 0, 0};
     const size_t esz3 = mixed ? sizeof(float) : sizeof(double);
@@ -882,13 +882,25 @@ int scfd_commit(scfd_ctx* c) {
                  need<unsigned long long>(2);
     const size_t nref = (size_t)(c->nimax + 4) * (c->njmax + 4) * c->np;
     bytes += need<double>((size_t)std::max(std::max(W, D), nY) * nref);
+    size_t records = 0;
     if (c->use_sw3)
-        bytes += need<char>(steps_total * wz.xs * esz3) + need<char>(steps_total * wz.cs * esz3) +
-                 need<long long>(step_off.size()) + need<int>(blks3.size()) + need<int>(strips3.size()) +
-                 need<int>(tasksf.size()) + need<int>(tasksb.size()) + need<double>((size_t)ntasks * xstride3);
+        records = need<char>(steps_total * wz.xs * esz3) + need<char>(steps_total * wz.cs * esz3) +
+                  need<long long>(step_off.size()) + need<int>(blks3.size()) + need<int>(strips3.size()) +
+                  need<int>(tasksf.size()) + need<int>(tasksb.size()) + need<double>((size_t)ntasks * xstride3);
     bytes += 64 * 256;
+    // a grid whose fields fit and whose records (320 B a cell with one species, 416 with
+    // nine) do not takes the generic sweeps, which need none
+    cudaError_t room = cudaMalloc(&c->arena, bytes + records);
+    if (room == cudaErrorMemoryAllocation && records > 0) {
+        cudaGetLastError();
+        records = 0;
+        c->use_sw3 = false;
+        room = cudaMalloc(&c->arena, bytes);
+    }
+    if (room != cudaSuccess)
+        return c->fail(SCFD_E_CUDA, std::string("cudaMalloc(&c->arena, bytes): ") + cudaGetErrorString(room));
+    bytes += records;
     c->arena_bytes = bytes;
-    CK(cudaMalloc(&c->arena, bytes));
     CK(cudaMemsetAsync(c->arena, 0, bytes, c->stream));
     char* p = c->arena;
     View& v = c->v;

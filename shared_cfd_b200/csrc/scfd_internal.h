@@ -273,7 +273,6 @@ int launch_chem_impl(const View& v, cudaStream_t s, int max_substeps, unsigned l
                      const ChemQueue& dq);
 int launch_step_end(const View& v, cudaStream_t s, double warn, double err);
 int launch_rms(const View& v, cudaStream_t s, double* partial, double* out);
-int launch_copy(double* dst, const double* src, long long n, cudaStream_t s);
 int launch_scalar_begin(const View& v, cudaStream_t s);
 int launch_to_f32(const View& v, cudaStream_t s);
 // reference layout <-> SoA slots (dir 0: ref -> soa, dir 1: soa -> ref_out)
