@@ -68,3 +68,40 @@ def test_preconditioned_sweep_edges(gpu, orc, scheme, n):
     assert rel_l2(case, got["q"], ref["q"]) <= 1e-10
     case.desc.precision = abi.PREC_MIXED
     assert rel_l2(case, run_case(case, gpu, 2)["q"], ref["q"]) <= 1e-4
+
+
+def test_records_without_room_take_the_generic_sweeps(gpu, monkeypatch):
+    """A grid whose fields fit on the device and whose strip records do not runs as it
+    does without them, bit for bit."""
+    import torch
+    from shared_cfd_b200.solver import Solver
+
+    monkeypatch.setenv("SCFD_AUTOTUNE", "0")
+    case = cases.flat_plate(768, 512)
+
+    def used():
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        s = Solver(case, gpu)
+        took = before - torch.cuda.mem_get_info()[0]
+        s.close()
+        return took
+
+    torch.cuda.init()
+    used()
+    full = used()
+    monkeypatch.setenv("SCFD_SWEEP_LEGACY", "1")
+    ref = run_case(case, gpu, 2)
+    fields = used()
+    monkeypatch.delenv("SCFD_SWEEP_LEGACY")
+    records = 8 * 40 * 768 * 512  # 40 doubles a cell
+    assert full - fields >= records
+    torch.cuda.empty_cache()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (full + fields) // 2, dtype=torch.uint8, device="cuda")
+    try:
+        got = run_case(case, gpu, 2)
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    assert got["stats"].status == 0
+    assert np.array_equal(got["q"][0], ref["q"][0])
