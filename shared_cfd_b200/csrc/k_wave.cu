@@ -162,6 +162,13 @@ struct WL {
     static constexpr size_t SMEM = UPC * UNIT + 16;
     static_assert(NY == 1 || NY == 8 || NY == 9, "components fit the lanes' slots");
     static_assert(UNIT % 16 == 0, "the second strip's rings are 16-byte aligned");
+    // arrivals of a phase of barrier k of the CTA's strip n, in the order of Unit: rfull, rdone,
+    // xfull, pempty, hempty, oful.  The top row's four lanes arrive on its own chunks (oful),
+    // and the first strip's on those that it writes into the second's ring (xfull).
+    static __host__ __device__ constexpr int arrivals(int n, int k) {
+        const int c = (k - 2 * PFB) / HS;
+        return k >= 2 * PFB && (c == 3 || (c == 0 && n == 1)) ? LPC : 1;
+    }
     // the component in slot s of lane sub, -1: none (a zero slot)
     static __host__ __device__ constexpr int comp(int sub, int s) {
         return NY == 1 ? sub : sub == 3 ? NY + s : 3 * sub + s < NY ? 3 * sub + s : -1;
@@ -621,15 +628,10 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kThreads, 1) k_wave
     // columns beyond a plane's last chunk are read (times alpha = 0) but never written
     for (int k = threadIdx.x; k < UPC * HS * HK * D4; k += kThreads)
         unit_at(k / (HS * HK * D4)).xin[k % (HS * HK * D4)] = RT(0);
-    if (threadIdx.x < UPC) {
-        const Unit q = unit_at(threadIdx.x);
-        for (int k = 0; k < 2 * PFB + 3 * HS; ++k) mbar_init(&q.rfull[k], 1);
-        for (int k = 0; k < HS; ++k) mbar_init(&q.oful[k], LPC);
-        // the second strip's chunks are written by the first strip's top row itself
-        if (threadIdx.x == 1)
-            for (int k = 0; k < HS; ++k) mbar_init(&q.xfull[k], LPC);
-        mbar_init_fence();
-    }
+    // every barrier once: a second init of a live mbarrier is undefined
+    for (int k = threadIdx.x; k < UPC * L::NBAR; k += kThreads)
+        mbar_init(&unit_at(k / L::NBAR).rfull[k % L::NBAR], L::arrivals(k / L::NBAR, k % L::NBAR));
+    mbar_init_fence();
     if (threadIdx.x == 0) {
         *s_bail = 0;
         *s_task = 0;

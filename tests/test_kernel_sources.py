@@ -1,0 +1,19 @@
+"""Rules of the kernels' sources that neither the compiler nor a run shows: what breaks
+them is undefined, whatever a device makes of it."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "shared_cfd_b200", "csrc")
+
+
+def source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def test_sweep_barriers_are_initialised_once():
+    """An mbarrier that is live may not be initialised again: one statement initialises
+    all of a sweep CTA's barriers, each with the arrivals of its phases."""
+    src = source("k_wave.cu")
+    assert len(re.findall(r"\bmbar_init\(", src)) == 1
+    assert re.search(r"for \(int k = threadIdx\.x; k < UPC \* L::NBAR; k \+= kThreads\)\s*mbar_init\(", src)
