@@ -1299,7 +1299,6 @@ int capture_steps(scfd_ctx* c, int n, cudaGraphExec_t* out, long long* launches)
 // Steps per replay of the long graph: the steps without an inner loop have 4 to 7 short
 // kernels, so that the gap between two graphs counts (Sod 15.0 -> 13.6 us a step).
 constexpr int kGraphSteps = 8;
-}  // namespace
 
 int step_once(scfd_ctx* c) {
     if (!c->tuned) {
@@ -1341,6 +1340,7 @@ int steps(scfd_ctx* c, int n) {
     }
     return 0;
 }
+}  // namespace
 
 int scfd_step(scfd_ctx* c, int step, scfd_stats* stats) {
     if (!c || !c->committed || !c->uploaded) return c ? c->fail(SCFD_E_STATE, "step before upload") : SCFD_E_ARG;
