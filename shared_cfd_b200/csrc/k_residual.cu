@@ -320,11 +320,8 @@ static void launch_t(const View& v, cudaStream_t s) {
     if (v.P.nact == 0) return;
     dim3 grid((nimax + TX - 1) / TX, (njmax + TY - 1) / TY, v.P.nact);
     const size_t smem = (size_t)(TY * (TX + 1) + (TY + 1) * TX) * v.D * sizeof(RT);
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaFuncSetAttribute(k_residual<RT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        attr_set = true;
-    }
+    // per device and its primary context: set before every launch (host only, cheap)
+    cudaFuncSetAttribute(k_residual<RT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     k_residual<RT, MODE><<<grid, NT, smem, s>>>(v);
 }
 

@@ -1127,14 +1127,6 @@ namespace {
 template <typename RT, int NY, int PRE, int DIR, int Q2D>
 int query_clusters() {
     using L = WL<RT, NY, PRE>;
-    if (cudaFuncSetAttribute(k_wave<RT, NY, PRE, DIR, Q2D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM) !=
-        cudaSuccess)
-        return 0;
-    if (cudaFuncSetAttribute(k_wave<RT, NY, PRE, DIR, Q2D>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-        cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(CL, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
@@ -1160,14 +1152,22 @@ int query_clusters() {
     return n;
 }
 
-// The device answers the same every time; the query takes milliseconds, so a process asks
-// once per kernel and device (the attributes that it sets stay set).
+// The kernel's attributes are set for every context: they go with the device's primary
+// context, which cudaDeviceReset ends.  The count of co-resident clusters is the device's
+// own, and its query takes milliseconds, so a process asks once per kernel and device.
 template <typename RT, int NY, int PRE, int DIR, int Q2D>
 int max_clusters_t() {
+    using L = WL<RT, NY, PRE>;
     static std::mutex m;
     static std::map<int, int> known;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    const auto kernel = k_wave<RT, NY, PRE, DIR, Q2D>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
     std::lock_guard<std::mutex> lock(m);
     const auto it = known.find(dev);
     if (it != known.end()) return it->second;
