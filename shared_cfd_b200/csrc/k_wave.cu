@@ -1176,21 +1176,25 @@ int max_clusters_t() {
     return n;
 }
 
+// of the two kernels that a context launches (each is loaded by its query): the forward
+// sweep of its dimension and the backward sweep
 template <typename RT, int NY, int PRE>
-int max_clusters_ny() {
-    int n = std::min(max_clusters_t<RT, NY, PRE, 0, 0>(), max_clusters_t<RT, NY, PRE, 1, 0>());
-    if constexpr (PRE == 0) n = std::min(n, max_clusters_t<RT, NY, PRE, 0, 1>());  // the preconditioned schemes are 2d
-    return n;
+int max_clusters_ny(bool q2d) {
+    int n = max_clusters_t<RT, NY, PRE, 1, 0>();
+    if constexpr (PRE == 0) {  // the preconditioned schemes are 2d
+        if (q2d) return std::min(n, max_clusters_t<RT, NY, PRE, 0, 1>());
+    }
+    return std::min(n, max_clusters_t<RT, NY, PRE, 0, 0>());
 }
 
 }  // namespace
 
-int wave_max_clusters(int ny, bool mixed, bool pre) {
-    if (pre) return ny != 1 ? 0 : mixed ? max_clusters_ny<float, 1, 1>() : max_clusters_ny<double, 1, 1>();
+int wave_max_clusters(int ny, bool mixed, bool pre, bool q2d) {
+    if (pre) return ny != 1 ? 0 : mixed ? max_clusters_ny<float, 1, 1>(q2d) : max_clusters_ny<double, 1, 1>(q2d);
     switch (ny) {
-        case 1: return mixed ? max_clusters_ny<float, 1, 0>() : max_clusters_ny<double, 1, 0>();
-        case 8: return mixed ? max_clusters_ny<float, 8, 0>() : max_clusters_ny<double, 8, 0>();
-        case 9: return mixed ? max_clusters_ny<float, 9, 0>() : max_clusters_ny<double, 9, 0>();
+        case 1: return mixed ? max_clusters_ny<float, 1, 0>(q2d) : max_clusters_ny<double, 1, 0>(q2d);
+        case 8: return mixed ? max_clusters_ny<float, 8, 0>(q2d) : max_clusters_ny<double, 8, 0>(q2d);
+        case 9: return mixed ? max_clusters_ny<float, 9, 0>(q2d) : max_clusters_ny<double, 9, 0>(q2d);
         default: return 0;
     }
 }

@@ -827,7 +827,7 @@ int scfd_commit(scfd_ctx* c) {
     const bool legacy = std::getenv("SCFD_SWEEP_LEGACY") != nullptr;
     const char* graph_env = std::getenv("SCFD_GRAPH");
     c->use_graph = !(graph_env && std::strcmp(graph_env, "0") == 0);
-    const int ncl_max = wz.xs > 0 && !legacy ? wave_max_clusters(nY, mixed, dual) : 0;
+    const int ncl_max = wz.xs > 0 && !legacy ? wave_max_clusters(nY, mixed, dual, c->d.dim == SCFD_DIM_Q2D) : 0;
     c->use_sw3 = wz.xs > 0 && !legacy && ncl_max > 0;
     std::vector<long long> step_off;
     std::vector<int> blks3, strips3, tasksf, tasksb;

@@ -253,7 +253,7 @@ int wave_pad_steps();                      // zero step blocks before and after 
 int wave_strips_per_task();
 int wave_handoff_chunk();                  // hand-off columns per chunk
 int wave_chunks(int ni);                   // hand-off chunks of a top row of ni columns
-int wave_max_clusters(int ny, bool mixed, bool pre); // co-resident clusters of the sweep kernel (0: none)
+int wave_max_clusters(int ny, bool mixed, bool pre, bool q2d); // co-resident clusters of the sweep kernels (0: none)
 int launch_wave(const View& v, cudaStream_t s, const Wave& w, int what, int inner);
 int launch_nr_update(const View& v, cudaStream_t s, const double* partials, int nstrips, int inner);
 // Cells whose CHEMEQ2 interval went to DVODE: k_chem queues them (the cell, the
