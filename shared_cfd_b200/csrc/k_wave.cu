@@ -29,7 +29,9 @@
 // 180 ns), of which the hand-off is about 10.
 //
 // A task is 256 consecutive rows of one plane at most, run by one thread-block
-// cluster of 16 CTAs with two strips each.  A strip's top row is staged in its
+// cluster of 16 CTAs with two strips each (128 rows and 8 CTAs, the largest portable
+// cluster, on a device or part of one that holds none of 16: its plane's top rows then
+// travel through global memory twice as often).  A strip's top row is staged in its
 // CTA's shared memory; every HK columns one bulk copy moves the chunk into the
 // next CTA's hand-off ring (distributed shared memory), completing a transaction count on
 // an mbarrier of the receiver, which releases consumed chunks with a remote arrive.  From a
@@ -74,8 +76,6 @@ namespace {
 constexpr int LPC = 4;   // lanes per cell
 constexpr int R = 32 / LPC;  // rows per strip
 constexpr int UPC = 2;   // strips per CTA
-constexpr int CL = 16;   // CTAs per cluster
-constexpr int SPT = CL * UPC;  // strips per task
 constexpr int HK = 4;    // hand-off columns per chunk
 constexpr int HS = 32;   // hand-off ring chunks
 constexpr int SPB = 8;   // steps per record slot (one wait and one release each)
@@ -583,7 +583,7 @@ struct CellStep {
 
 // one CTA per SM (its shared memory)
 template <typename RT, int NY, int PRE, int DIR, int Q2D>
-__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kThreads, 1) k_wave(View v, WaveArgs a) {
+__global__ void __launch_bounds__(kThreads, 1) k_wave(View v, WaveArgs a) {
     using L = WL<RT, NY, PRE>;
     constexpr int XS = L::XS, CSZ = L::CS, D4 = L::D4, K = L::K, PFB = L::PFB;
     constexpr unsigned CHUNK_BYTES = HK * D4 * sizeof(RT);
@@ -1097,7 +1097,7 @@ k_unpack(View v, const int2* blk, const int4* strips, const long long* step_off,
 // host side
 // ---------------------------------------------------------------------------
 int wave_pad_steps() { return kPadSteps; }
-int wave_strips_per_task() { return SPT; }
+int wave_strips_per_task(int cl) { return cl * UPC; }
 int wave_handoff_chunk() { return HK; }
 int wave_chunks(int ni) { return chunks_of(ni); }
 int wave_rows() { return R; }
@@ -1124,42 +1124,24 @@ WaveSizes wave_sizes(int ny, bool mixed, bool pre) {
 
 namespace {
 
-template <typename RT, int NY, int PRE, int DIR, int Q2D>
-int query_clusters() {
-    using L = WL<RT, NY, PRE>;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(CL, 1, 1);
-    cfg.blockDim = dim3(kThreads, 1, 1);
-    cfg.dynamicSmemBytes = L::SMEM;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = CL;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    // the kernel carries its cluster shape; some runtimes want it repeated
-    // in the query's attributes, others reject that
-    int n = 0;
-    cfg.numAttrs = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_wave<RT, NY, PRE, DIR, Q2D>, &cfg) == cudaSuccess && n > 0) return n;
-    cudaGetLastError();
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_wave<RT, NY, PRE, DIR, Q2D>, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return n;
+cudaLaunchAttribute cluster_of(int cl) {
+    cudaLaunchAttribute a{};
+    a.id = cudaLaunchAttributeClusterDimension;
+    a.val.clusterDim.x = cl;
+    a.val.clusterDim.y = 1;
+    a.val.clusterDim.z = 1;
+    return a;
 }
 
 // The kernel's attributes are set for every context: they go with the device's primary
 // context, which cudaDeviceReset ends.  The count of co-resident clusters is the device's
-// own, and its query takes milliseconds, so a process asks once per kernel and device.
+// own, and its query takes milliseconds, so a process asks once per kernel, device and
+// cluster size.
 template <typename RT, int NY, int PRE, int DIR, int Q2D>
-int max_clusters_t() {
+int max_clusters_t(int cl) {
     using L = WL<RT, NY, PRE>;
     static std::mutex m;
-    static std::map<int, int> known;
+    static std::map<std::pair<int, int>, int> known;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     const auto kernel = k_wave<RT, NY, PRE, DIR, Q2D>;
@@ -1169,32 +1151,43 @@ int max_clusters_t() {
         return 0;
     }
     std::lock_guard<std::mutex> lock(m);
-    const auto it = known.find(dev);
+    const auto it = known.find({dev, cl});
     if (it != known.end()) return it->second;
-    const int n = query_clusters<RT, NY, PRE, DIR, Q2D>();
-    if (n > 0) known[dev] = n;
+    cudaLaunchAttribute attr = cluster_of(cl);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cl, 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = L::SMEM;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (n > 0) known[{dev, cl}] = n;
     return n;
 }
 
 // of the two kernels that a context launches (each is loaded by its query): the forward
 // sweep of its dimension and the backward sweep
 template <typename RT, int NY, int PRE>
-int max_clusters_ny(bool q2d) {
-    int n = max_clusters_t<RT, NY, PRE, 1, 0>();
+int max_clusters_ny(bool q2d, int cl) {
+    int n = max_clusters_t<RT, NY, PRE, 1, 0>(cl);
     if constexpr (PRE == 0) {  // the preconditioned schemes are 2d
-        if (q2d) return std::min(n, max_clusters_t<RT, NY, PRE, 0, 1>());
+        if (q2d) return std::min(n, max_clusters_t<RT, NY, PRE, 0, 1>(cl));
     }
-    return std::min(n, max_clusters_t<RT, NY, PRE, 0, 0>());
+    return std::min(n, max_clusters_t<RT, NY, PRE, 0, 0>(cl));
 }
 
 }  // namespace
 
-int wave_max_clusters(int ny, bool mixed, bool pre, bool q2d) {
-    if (pre) return ny != 1 ? 0 : mixed ? max_clusters_ny<float, 1, 1>(q2d) : max_clusters_ny<double, 1, 1>(q2d);
+int wave_max_clusters(int ny, bool mixed, bool pre, bool q2d, int cl) {
+    if (pre) return ny != 1 ? 0 : mixed ? max_clusters_ny<float, 1, 1>(q2d, cl) : max_clusters_ny<double, 1, 1>(q2d, cl);
     switch (ny) {
-        case 1: return mixed ? max_clusters_ny<float, 1, 0>(q2d) : max_clusters_ny<double, 1, 0>(q2d);
-        case 8: return mixed ? max_clusters_ny<float, 8, 0>(q2d) : max_clusters_ny<double, 8, 0>(q2d);
-        case 9: return mixed ? max_clusters_ny<float, 9, 0>(q2d) : max_clusters_ny<double, 9, 0>(q2d);
+        case 1: return mixed ? max_clusters_ny<float, 1, 0>(q2d, cl) : max_clusters_ny<double, 1, 0>(q2d, cl);
+        case 8: return mixed ? max_clusters_ny<float, 8, 0>(q2d, cl) : max_clusters_ny<double, 8, 0>(q2d, cl);
+        case 9: return mixed ? max_clusters_ny<float, 9, 0>(q2d, cl) : max_clusters_ny<double, 9, 0>(q2d, cl);
         default: return 0;
     }
 }
@@ -1207,7 +1200,15 @@ void sweep_launch(const View& v, cudaStream_t s, const Wave& w) {
     WaveArgs a{DIR == 0 ? w.tasks_f : w.tasks_b, w.ntasks,    w.step_off, w.X, w.C, w.xfer, w.xstride,
                w.progress + (DIR == 0 ? 0 : w.ntasks), w.tickets + (DIR == 0 ? 0 : 1)};
     const int ncl = w.nclusters < w.ntasks ? w.nclusters : w.ntasks;
-    k_wave<RT, NY, PRE, DIR, Q2D><<<ncl * CL, kThreads, L::SMEM, s>>>(v, a);
+    cudaLaunchAttribute attr = cluster_of(w.cluster);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ncl * w.cluster, 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = L::SMEM;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_wave<RT, NY, PRE, DIR, Q2D>, v, a);
 }
 
 template <typename RT, int NY, int PRE>

@@ -55,6 +55,7 @@ struct scfd_ctx {
     int valstride = SCFD_BC_MAXVAL + 2;
     // cluster-wavefront sweeps over strip records (k_wave.cu)
     bool use_sw3 = false;
+    const char* no_sw3 = "";  // why not
     Wave sw3{};
     // chemistry
     unsigned long long* d_counter = nullptr;
@@ -827,13 +828,23 @@ int scfd_commit(scfd_ctx* c) {
     const bool legacy = std::getenv("SCFD_SWEEP_LEGACY") != nullptr;
     const char* graph_env = std::getenv("SCFD_GRAPH");
     c->use_graph = !(graph_env && std::strcmp(graph_env, "0") == 0);
-    const int ncl_max = wz.xs > 0 && !legacy ? wave_max_clusters(nY, mixed, dual, c->d.dim == SCFD_DIM_Q2D) : 0;
-    c->use_sw3 = wz.xs > 0 && !legacy && ncl_max > 0;
+    // clusters of 16 CTAs, of 8 (which every device part can hold) where none of 16 fits;
+    // SCFD_SWEEP_CLUSTER=8 takes 8 anywhere
+    const char* cluster_env = std::getenv("SCFD_SWEEP_CLUSTER");
+    const int cluster_max = cluster_env && std::strcmp(cluster_env, "8") == 0 ? 8 : 16;
+    int ncl_max = 0, cluster = 0;
+    if (wz.xs > 0 && !legacy)
+        for (int cl = cluster_max; cl >= 8 && ncl_max == 0; cl /= 2) {
+            cluster = cl;
+            ncl_max = wave_max_clusters(nY, mixed, dual, c->d.dim == SCFD_DIM_Q2D, cl);
+        }
+    c->use_sw3 = ncl_max > 0;
+    c->no_sw3 = !impl ? "" : legacy ? "SCFD_SWEEP_LEGACY" : wz.xs == 0 ? "species count" : "no cluster of 8 CTAs fits";
     std::vector<long long> step_off;
     std::vector<int> blks3, strips3, tasksf, tasksb;
     long long steps_total = 0;
     if (c->use_sw3) {
-        const int pad = wave_pad_steps(), tpc = wave_strips_per_task(), rows = wave_rows();
+        const int pad = wave_pad_steps(), tpc = wave_strips_per_task(cluster), rows = wave_rows();
         int fs = 0;
         for (int pl = 0; pl < c->np; ++pl) {
             if (!c->own(pl)) continue;
@@ -895,6 +906,7 @@ int scfd_commit(scfd_ctx* c) {
         cudaGetLastError();
         records = 0;
         c->use_sw3 = false;
+        c->no_sw3 = "no memory for the strip records";
         room = cudaMalloc(&c->arena, bytes);
     }
     if (room != cudaSuccess)
@@ -986,6 +998,7 @@ int scfd_commit(scfd_ctx* c) {
         w3.tasks_b = reinterpret_cast<const int4*>(tb);
         w3.ntasks = ntasks;
         w3.nclusters = std::min(ntasks, ncl_max);
+        w3.cluster = cluster;
         w3.xstride = xstride3;
         w3.progress = c->d_progress;
         w3.tickets = c->d_tickets;
@@ -1797,11 +1810,13 @@ int scfd_tuning(scfd_ctx* c, char* json, int len) {
     std::string rep = c->tune_report;
     char sw[160];
     if (c->use_sw3)
-        std::snprintf(sw, sizeof(sw), "\"sweep\": {\"kind\": \"cluster wavefront\", \"tasks\": %d, \"clusters\": %d}",
-                      c->sw3.ntasks, c->sw3.nclusters);
+        std::snprintf(sw, sizeof(sw),
+                      "\"sweep\": {\"kind\": \"cluster wavefront\", \"tasks\": %d, \"clusters\": %d, \"cluster_ctas\": %d}",
+                      c->sw3.ntasks, c->sw3.nclusters, c->sw3.cluster);
+    else if (c->d.scheme == SCFD_SCHEME_EULER)
+        std::snprintf(sw, sizeof(sw), "\"sweep\": {\"kind\": \"none\"}");
     else
-        std::snprintf(sw, sizeof(sw), "\"sweep\": {\"kind\": \"%s\"}",
-                      c->d.scheme == SCFD_SCHEME_EULER ? "none" : "generic");
+        std::snprintf(sw, sizeof(sw), "\"sweep\": {\"kind\": \"generic\", \"reason\": \"%s\"}", c->no_sw3);
     const size_t close = rep.rfind('}');
     if (close != std::string::npos) rep = rep.substr(0, close) + (rep.size() > 2 ? ", " : "") + sw + "}";
     std::snprintf(json, (size_t)len, "%s", rep.c_str());

@@ -233,10 +233,11 @@ struct Wave {
     const int4* strips;         // per forward strip (plane, s, strip, 0): pack / unpack
     const int2* blk;            // pack/unpack blocks: (strip, first step)
     int nblk;
-    const int4* tasks_f;        // tasks of up to 256 rows (plane, first strip, strips, strip 0's index)
+    const int4* tasks_f;        // tasks of a cluster's rows (plane, first strip, strips, strip 0's index)
     const int4* tasks_b;        // backward order
     int ntasks;
     int nclusters;              // clusters launched (at most ntasks)
+    int cluster;                // CTAs per cluster
     void* xfer;                 // per task: published hand-off columns
     long long xstride;          // elements per task
     int* progress;              // 2*ntasks
@@ -250,10 +251,11 @@ struct WaveSizes {
 WaveSizes wave_sizes(int ny, bool mixed, bool pre);  // xs = 0 if there is no sweep
 int wave_rows();                           // rows per strip
 int wave_pad_steps();                      // zero step blocks before and after each strip
-int wave_strips_per_task();
+int wave_strips_per_task(int cl);           // of a cluster of cl CTAs
 int wave_handoff_chunk();                  // hand-off columns per chunk
 int wave_chunks(int ni);                   // hand-off chunks of a top row of ni columns
-int wave_max_clusters(int ny, bool mixed, bool pre, bool q2d); // co-resident clusters of the sweep kernels (0: none)
+// co-resident clusters of cl CTAs of the sweep kernels (0: none)
+int wave_max_clusters(int ny, bool mixed, bool pre, bool q2d, int cl);
 int launch_wave(const View& v, cudaStream_t s, const Wave& w, int what, int inner);
 int launch_nr_update(const View& v, cudaStream_t s, const double* partials, int nstrips, int inner);
 // Cells whose CHEMEQ2 interval went to DVODE: k_chem queues them (the cell, the
