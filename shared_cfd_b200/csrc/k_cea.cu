@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(128, 2) k_cea_hptp(const CeaTab<NS, NE, NSEC>*
                                                     double* __restrict__ n_io, HpTpOut out,
                                                     unsigned long long* __restrict__ fails) {
     using Tab = CeaTab<NS, NE, NSEC>;
-    extern __shared__ double smem_tab[];
+    extern __shared__ __align__(16) double smem_tab[];
     {
         const double* src = reinterpret_cast<const double*>(gtab);
         for (int k = threadIdx.x; k < (int)(sizeof(Tab) / sizeof(double)); k += blockDim.x) smem_tab[k] = src[k];

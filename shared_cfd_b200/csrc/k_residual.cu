@@ -213,7 +213,7 @@ __device__ void face_flux(const View& v, int p, int i, int j, RT* fout) {
 
 template <typename RT, int MODE>
 __global__ void __launch_bounds__(NT) k_residual(View v) {
-    extern __shared__ unsigned char smraw[];
+    extern __shared__ __align__(16) unsigned char smraw[];
     RT* FI = reinterpret_cast<RT*>(smraw);
     const int D = v.D, nY = v.nY;
     RT* FJ = FI + TY * (TX + 1) * D;

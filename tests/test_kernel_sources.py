@@ -17,3 +17,15 @@ def test_sweep_barriers_are_initialised_once():
     src = source("k_wave.cu")
     assert len(re.findall(r"\bmbar_init\(", src)) == 1
     assert re.search(r"for \(int k = threadIdx\.x; k < UPC \* L::NBAR; k \+= kThreads\)\s*mbar_init\(", src)
+
+
+def test_dynamic_shared_memory_is_declared_aligned():
+    """Every kernel reads its dynamic shared memory as doubles or 16-byte vectors (k_cea's
+    species tables as double2 in all its kernels), so each declares that alignment."""
+    found = 0
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            for decl in re.findall(r"extern __shared__[^;]*;", source(name)):
+                found += 1
+                assert re.search(r"__align__\((16|32|64|128)\)", decl), (name, decl)
+    assert found >= 7
