@@ -590,7 +590,10 @@ __global__ void __launch_bounds__(kCeaThreads, MINB) k_cea(const CeaTab<NS, NE, 
                 const double phi = 0.25 * (f * f) * t.wsq[i][j];
                 denom += nfit[j] * phi;
             }
-            mu += scfd::div_pos(nfit[i] * (sq[i] * sq[i]), denom);
+            // far below the fits' range a fit's exponential underflows and the sum over the others
+            // overflows: the term is 0 then, outside div_pos's domain
+            const double num = nfit[i] * (sq[i] * sq[i]);
+            mu += denom < 1e290 ? scfd::div_pos(num, denom) : num / denom;
         }
         out.mu[c] = mu * 1e-7;
     }
