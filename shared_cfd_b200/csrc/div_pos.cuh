@@ -3,7 +3,7 @@
 
 namespace scfd {
 
-// a / b for a positive normal b, without branches: the IEEE division's
+// a / b for an ordinary b of either sign (normal, with a normal reciprocal), without branches: the IEEE division's
 // out-of-line slow path keeps the many independent quotients of a thread apart,
 // these overlap.  Newton-Raphson on the reciprocal from the hardware's
 // approximate reciprocal y0 (rcp.approx.ftz, about 23 bits): FP64 takes one
@@ -11,9 +11,10 @@ namespace scfd {
 // e^3), FP32 one second-order step y1 = y0 (1 + e); then q0 = a y1 and
 // Markstein's remainder correction q = q0 + (a - b q0) y1.  The result is
 // within one unit in the last place of a / b (tests/test_division.py checks the
-// steps in exact arithmetic from seeds 2^-21 off).  A zero, subnormal, infinite
-// or negative b is outside its domain; each kernel that uses it states which
-// denominators it gives it.
+// steps in exact arithmetic from seeds 2^-21 off, tests/test_division_domain.py for
+// negative and very small b; a sign goes through every step unchanged).  A zero,
+// subnormal or infinite b, or an infinite quotient, is outside its domain and gives NaN;
+// each kernel that uses it states which denominators it gives it.
 __device__ __forceinline__ double div_pos(double a, double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));

@@ -90,6 +90,13 @@ __device__ __forceinline__ int tsection(const double* thi, double tlo, int nsec,
     return nsec - 1;
 }
 
+// The quotients of k_cea and the tables' vectors go through div_pos.  Its denominators:
+// T^2 and RU T (a step changes T by 0.4 in the logarithm at most, 500 steps by e^200, so
+// they are ordinary from any T between 1e-60 and 1e60; at others vert is not finite and the
+// cell ends singular, or as it would), the pivots (of either sign, 1e-30 or more: below
+// that the solution is thrown away), the molecular weights, the sum of n,
+// cp/R - sum n (above 0 for every fit), Y's element sums + 1e-300 and,
+// where it is finite, the Wilke sum (above the term's own n).
 // x / D for a small whole number D: the product with its reciprocal and Markstein's
 // remainder correction, without the division's out-of-line slow path
 template <int D>
