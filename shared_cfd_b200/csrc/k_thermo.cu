@@ -355,6 +355,7 @@ __global__ void __launch_bounds__(256, 2) k_thermo_fixed(View v, int flags) {
     if (PRO) prologue(v, flags, in, p, i, j);
 }
 
+// any mechanism
 __device__ __forceinline__ void thermo_any(const View& v, long long c) {
     const long long N = v.ncell;
     const int nY = v.nY, D = v.D;
@@ -374,22 +375,6 @@ __device__ __forceinline__ void thermo_any(const View& v, long long c) {
     for (int k = 0; k < nY; ++k) w[(k + 4) * N + c] = q[k * N + c] * tmp;
     const double qE = q[(nY + 2) * N + c];
     const double ei = qE / rho - 0.5 * (u * u + vv * vv);
-    if (v.thermo == SCFD_THERMO_IDEAL) {
-        const double kg = v.kappa, Rg = v.rgas;
-        const double T = ei * (kg - 1.0) / Rg;
-        const double pr = rho * Rg * T;
-        w[3 * N + c] = pr;
-        w[ig * N + c] = kg;
-        w[iht * N + c] = (qE + pr) / rho;
-        if (v.mu_model == SCFD_MU_SUTHERLAND)
-            w[imu * N + c] = v.suth_mu0 * pow(T / v.suth_t0, 1.5) * (v.suth_t0 + v.suth_s) / (T + v.suth_s);
-        else
-            w[imu * N + c] = rho * v.nu_gas;
-        w[iR * N + c] = Rg;
-        for (int k = 0; k < nY; ++k) v.DHi[k * N + c] = 0.0;
-        v.vhi[c] = kg / (kg - 1.0) * Rg * T;
-        return;
-    }
     double vrho[kMaxSpecies], DH[kMaxSpecies], vh[kMaxSpecies];
     for (int k = 0; k < nY; ++k) vrho[k] = q[k * N + c];
     double T = w[3 * N + c] / (rho * w[iR * N + c]);
@@ -420,8 +405,8 @@ __global__ void __launch_bounds__(256) k_thermo(View v, int flags) {
     if (PRO) prologue(v, flags, in, p, i, j);
 }
 
-// k_thermo for the ideal gas (one species), straight through: every load first, the
-// prologue from registers.  The generic form read back what it had just written (sqrt of
+// The ideal gas (one species), straight through: every load first, the prologue from
+// registers.  The form over any number of species read back what it had just written (sqrt of
 // gamma p / rho, q for the copies) and waited for each load of its species loops: 6.8 us
 // for 1600 cells and 10.4 us for 197 k with the prologue.  Same arithmetic.
 template <bool PRO>
@@ -499,7 +484,7 @@ int launch_thermo(const View& v, cudaStream_t s, int cells_per_plane_max, int pr
     if (v.thermo != SCFD_THERMO_IDEAL && v.chem.ns == 9 && v.nY == 9 && v.chem.nt <= 9) {
         if (prologue) k_thermo_fixed<9, true><<<grid, bs, 0, s>>>(v, prologue);
         else k_thermo_fixed<9, false><<<grid, bs, 0, s>>>(v, 0);
-    } else if (v.thermo == SCFD_THERMO_IDEAL && v.nY == 1) {
+    } else if (v.thermo == SCFD_THERMO_IDEAL) {  // one species (scfd_create)
         if (prologue) k_thermo_ideal<true><<<grid, bs, 0, s>>>(v, prologue);
         else k_thermo_ideal<false><<<grid, bs, 0, s>>>(v, 0);
     } else {
