@@ -76,6 +76,8 @@ struct scfd_ctx {
     int eager_steps = 0;
     cudaGraphExec_t graph = nullptr, graph_n = nullptr;  // one step; kGraphSteps steps
     long long graph_launches = 0, graph_n_launches = 0;
+    long long run_steps = 0;   // steps of runs that a long graph could have taken
+    bool long_graph = true;    // false: it could not be built
     std::vector<cudaEvent_t> ev_pool;
     size_t ev_used = 0;
     std::vector<std::pair<int, size_t>> ev_marks;  // kind, index of the start event
@@ -1310,8 +1312,11 @@ int capture_steps(scfd_ctx* c, int n, cudaGraphExec_t* out, long long* launches)
 }
 
 // Steps per replay of the long graph: the steps without an inner loop have 4 to 7 short
-// kernels, so that the gap between two graphs counts (Sod 15.0 -> 13.6 us a step).
+// kernels, so that the gap between two graphs counts (Sod 15.3 -> 13.4 us a step).
 constexpr int kGraphSteps = 8;
+// Building it takes 230 to 390 us and a step in it saves 1.4 to 3 us (400 x 4 to 256 x 128
+// cells, explicit, LU-SGS and preconditioned LU-SGS), which is even after 120 to 280 steps.
+constexpr long long kLongGraphAfter = 160;
 
 int step_once(scfd_ctx* c) {
     if (!c->tuned) {
@@ -1333,13 +1338,18 @@ int step_once(scfd_ctx* c) {
 
 // n steps, several to a graph where that pays
 int steps(scfd_ctx* c, int n) {
-    // a long graph is built for a run that replays it a few times
-    const bool many = (c->graph_n || n >= 4 * kGraphSteps) && !dual_time_scheme(c->d.scheme) && !c->profiling;
+    // the long graph is built once a run, or the context's runs so far, would have paid for it
+    if (n >= kGraphSteps) c->run_steps += n;
+    const bool many = c->long_graph && !dual_time_scheme(c->d.scheme) && !c->profiling &&
+                      (c->graph_n || c->run_steps >= kLongGraphAfter);
     while (n > 0) {
-        if (many && c->graph && n >= kGraphSteps) {
-            if (!c->graph_n) {
-                const int st = capture_steps(c, kGraphSteps, &c->graph_n, &c->graph_n_launches);
-                if (st) return st;
+        if (many && c->graph && n >= kGraphSteps && c->long_graph) {
+            if (!c->graph_n && capture_steps(c, kGraphSteps, &c->graph_n, &c->graph_n_launches)) {
+                // without it every step has its own launch, as before
+                cudaGetLastError();
+                c->err.clear();
+                c->long_graph = false;
+                continue;
             }
             CK(cudaGraphLaunch(c->graph_n, c->stream));
             c->launches += c->graph_n_launches;
@@ -1817,8 +1827,9 @@ int scfd_tuning(scfd_ctx* c, char* json, int len) {
         std::snprintf(sw, sizeof(sw), "\"sweep\": {\"kind\": \"none\"}");
     else
         std::snprintf(sw, sizeof(sw), "\"sweep\": {\"kind\": \"generic\", \"reason\": \"%s\"}", c->no_sw3);
+    const std::string graph = c->graph ? ", \"graph_steps\": " + std::to_string(c->graph_n ? kGraphSteps : 1) : "";
     const size_t close = rep.rfind('}');
-    if (close != std::string::npos) rep = rep.substr(0, close) + (rep.size() > 2 ? ", " : "") + sw + "}";
+    if (close != std::string::npos) rep = rep.substr(0, close) + (rep.size() > 2 ? ", " : "") + sw + graph + "}";
     std::snprintf(json, (size_t)len, "%s", rep.c_str());
     return (int)rep.size() < len ? 0 : SCFD_E_ARG;
 }
