@@ -151,14 +151,15 @@ __global__ void k_step_end(View v, double warn, double err) {
 
 // Field transposes between the reference layout f(1:nk,-1:nimax+2,-1:njmax+2,Nplane)
 // (component fastest) and the structure-of-arrays cell slots: one thread per
-// reference cell; dir 0 scatters ref -> SoA, dir 1 gathers SoA -> ref (cells
-// beyond a smaller plane's ghost layers are written as zero).
-__global__ void k_ref_soa(Planes P, long long N, int nk, int IX, int JX, long long nref, const double* ref,
+// reference cell of first .. first + n - 1, whose values ref / ref_out hold; dir 0 scatters
+// ref -> SoA, dir 1 gathers SoA -> ref (cells beyond a smaller plane's ghost layers are
+// written as zero).
+__global__ void k_ref_soa(Planes P, long long N, int nk, int IX, int JX, long long first, long long n, const double* ref,
                           double* soa, double* ref_out, int dir) {
-    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < nref;
+    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n;
          idx += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(idx % IX) - 1;
-        const long long r = idx / IX;
+        const int i = (int)((first + idx) % IX) - 1;
+        const long long r = (first + idx) / IX;
         const int j = (int)(r % JX) - 1, p = (int)(r / JX);
         const bool in = i <= P.ni[p] + 2 && j <= P.nj[p] + 2;
         const long long c = in ? cidx(P, p, i, j) : 0;
@@ -171,11 +172,10 @@ __global__ void k_ref_soa(Planes P, long long N, int nk, int IX, int JX, long lo
     }
 }
 
-int launch_ref_soa(const View& v, cudaStream_t s, int nk, int IX, int JX, const double* ref, double* soa,
-                   double* ref_out, int dir) {
-    const long long nref = (long long)IX * JX * v.P.np;
-    const int blocks = (int)std::min<long long>((nref + 255) / 256, 148LL * 16);
-    k_ref_soa<<<blocks, 256, 0, s>>>(v.P, v.ncell, nk, IX, JX, nref, ref, soa, ref_out, dir);
+int launch_ref_soa(const View& v, cudaStream_t s, int nk, int IX, int JX, long long first, long long n, const double* ref,
+                   double* soa, double* ref_out, int dir) {
+    const int blocks = (int)std::min<long long>((n + 255) / 256, 148LL * 16);
+    k_ref_soa<<<blocks, 256, 0, s>>>(v.P, v.ncell, nk, IX, JX, first, n, ref, soa, ref_out, dir);
     return 1;
 }
 

@@ -18,6 +18,8 @@ using namespace scfd;
 
 // bytes of each pinned chunk of the host <-> device copies (two chunks per context)
 constexpr size_t kRingChunk = 32ull << 20;
+// the device staging of a field in the reference layout where a whole field does not fit
+constexpr size_t kRefChunk = 64ull << 20;
 
 struct scfd_ctx {
     scfd_desc d{};
@@ -64,7 +66,8 @@ struct scfd_ctx {
     double* d_rms_partial = nullptr;
     double* d_rms_out = nullptr;
     // pinned staging for transfers
-    double* d_ref = nullptr;  // device staging of one field in the reference layout
+    double* d_ref = nullptr;  // device staging of one field, or a part of it, in the reference layout
+    size_t ref_len = 0;       // its doubles
     void* h_ring[2] = {nullptr, nullptr};  // pinned chunks of the host <-> device copies
     cudaEvent_t ring_ev[2] = {nullptr, nullptr};
     long long launches = 0;
@@ -894,26 +897,37 @@ int scfd_commit(scfd_ctx* c) {
         bytes += need<long long>(dq_cap) + need<double>(dq_cap) + need<double>((size_t)dq_cap * (c->chem.ns + 1)) +
                  need<unsigned long long>(2);
     const size_t nref = (size_t)(c->nimax + 4) * (c->njmax + 4) * c->np;
-    bytes += need<double>((size_t)std::max(std::max(W, D), nY) * nref);
+    const size_t ref_all = (size_t)std::max(std::max(W, D), nY) * nref;
     size_t records = 0;
     if (c->use_sw3)
         records = need<char>(steps_total * wz.xs * esz3) + need<char>(steps_total * wz.cs * esz3) +
                   need<long long>(step_off.size()) + need<int>(blks3.size()) + need<int>(strips3.size()) +
                   need<int>(tasksf.size()) + need<int>(tasksb.size()) + need<double>((size_t)ntasks * xstride3);
     bytes += 64 * 256;
-    // a grid whose fields fit and whose records (320 B a cell with one species, 416 with
-    // nine) do not takes the generic sweeps, which need none
-    cudaError_t room = cudaMalloc(&c->arena, bytes + records);
-    if (room == cudaErrorMemoryAllocation && records > 0) {
+    // What a large grid does without where memory is short: first the staging of a whole
+    // field (72 B a cell with one species, 136 with nine; a part of it takes the copies to
+    // the host in parts), then the strip records (320 and 416 B), for the generic sweeps.
+    // SCFD_MEM_LIMIT: as if the device had no more than that (bytes).
+    const char* limit_env = std::getenv("SCFD_MEM_LIMIT");
+    const unsigned long long limit = limit_env ? std::strtoull(limit_env, nullptr, 10) : 0;
+    const size_t ref_part = std::min(ref_all, kRefChunk / sizeof(double));
+    const struct { size_t ref, records; } tries[3] = {{ref_all, records}, {ref_part, records}, {ref_part, 0}};
+    cudaError_t room = cudaErrorMemoryAllocation;
+    size_t total = 0;
+    for (const auto& t : tries) {
+        total = bytes + need<double>(t.ref) + t.records;
+        c->ref_len = t.ref;
+        if (t.records == 0 && c->use_sw3) {
+            c->use_sw3 = false;
+            c->no_sw3 = "no memory for the strip records";
+        }
+        room = limit > 0 && total > limit ? cudaErrorMemoryAllocation : cudaMalloc(&c->arena, total);
+        if (room != cudaErrorMemoryAllocation) break;
         cudaGetLastError();
-        records = 0;
-        c->use_sw3 = false;
-        c->no_sw3 = "no memory for the strip records";
-        room = cudaMalloc(&c->arena, bytes);
     }
     if (room != cudaSuccess)
-        return c->fail(SCFD_E_CUDA, std::string("cudaMalloc(&c->arena, bytes): ") + cudaGetErrorString(room));
-    bytes += records;
+        return c->fail(SCFD_E_CUDA, std::string("cudaMalloc(&c->arena, total): ") + cudaGetErrorString(room));
+    bytes = total;
     c->arena_bytes = bytes;
     CK(cudaMemsetAsync(c->arena, 0, bytes, c->stream));
     char* p = c->arena;
@@ -972,7 +986,7 @@ int scfd_commit(scfd_ctx* c) {
     }
     c->d_rms_partial = carve<double>(p, nrec);
     c->d_rms_out = carve<double>(p, 1);
-    c->d_ref = carve<double>(p, (size_t)std::max(std::max(W, D), nY) * nref);
+    c->d_ref = carve<double>(p, c->ref_len);
     for (int b = 0; b < 2; ++b) {
         CK(cudaMallocHost(&c->h_ring[b], kRingChunk));
         CK(cudaEventCreateWithFlags(&c->ring_ev[b], cudaEventDisableTiming));
@@ -1125,22 +1139,31 @@ static int d2h_pipelined(scfd_ctx* c, void* host, const void* dev, size_t bytes)
 }
 
 // The reference-layout arrays cross PCIe unchanged into a device staging
-// buffer (d_ref) and are transposed to / from the cell slots on the GPU.
+// buffer (d_ref) and are transposed to / from the cell slots on the GPU, in as many parts
+// as the buffer asks for.
 static int upload_field(scfd_ctx* c, const double* ref, int nk, double* dev) {
     const int IX = c->nimax + 4, JX = c->njmax + 4;
-    const size_t bytes = sizeof(double) * (size_t)nk * IX * JX * c->np;
-    int st = h2d_pipelined(c, c->d_ref, ref, bytes);
-    if (st) return st;
-    launch_ref_soa(c->v, c->stream, nk, IX, JX, c->d_ref, dev, nullptr, 0);
-    CK(cudaGetLastError());
+    const long long nref = (long long)IX * JX * c->np, part = (long long)(c->ref_len / nk);
+    for (long long at = 0; at < nref; at += part) {
+        const long long n = std::min(part, nref - at);
+        int st = h2d_pipelined(c, c->d_ref, ref + at * nk, sizeof(double) * (size_t)(n * nk));
+        if (st) return st;
+        launch_ref_soa(c->v, c->stream, nk, IX, JX, at, n, c->d_ref, dev, nullptr, 0);
+        CK(cudaGetLastError());
+    }
     return 0;
 }
 static int download_field(scfd_ctx* c, const double* dev, int nk, double* ref) {
     const int IX = c->nimax + 4, JX = c->njmax + 4;
-    const size_t bytes = sizeof(double) * (size_t)nk * IX * JX * c->np;
-    launch_ref_soa(c->v, c->stream, nk, IX, JX, nullptr, const_cast<double*>(dev), c->d_ref, 1);
-    CK(cudaGetLastError());
-    return d2h_pipelined(c, ref, c->d_ref, bytes);
+    const long long nref = (long long)IX * JX * c->np, part = (long long)(c->ref_len / nk);
+    for (long long at = 0; at < nref; at += part) {
+        const long long n = std::min(part, nref - at);
+        launch_ref_soa(c->v, c->stream, nk, IX, JX, at, n, nullptr, const_cast<double*>(dev), c->d_ref, 1);
+        CK(cudaGetLastError());
+        int st = d2h_pipelined(c, ref + at * nk, c->d_ref, sizeof(double) * (size_t)(n * nk));
+        if (st) return st;
+    }
+    return 0;
 }
 
 int scfd_upload(scfd_ctx* c, const double* q, const double* w, const double* vhi, double tt) {
@@ -1827,6 +1850,10 @@ int scfd_tuning(scfd_ctx* c, char* json, int len) {
         std::snprintf(sw, sizeof(sw), "\"sweep\": {\"kind\": \"none\"}");
     else
         std::snprintf(sw, sizeof(sw), "\"sweep\": {\"kind\": \"generic\", \"reason\": \"%s\"}", c->no_sw3);
+    if (c->arena)
+        rep.insert(rep.rfind('}'), std::string(rep.size() > 2 ? ", " : "") + "\"memory\": {\"arena_bytes\": " +
+                                       std::to_string(c->arena_bytes) + ", \"staging_bytes\": " +
+                                       std::to_string(c->ref_len * sizeof(double)) + "}");
     const std::string graph = c->graph ? ", \"graph_steps\": " + std::to_string(c->graph_n ? kGraphSteps : 1) : "";
     const size_t close = rep.rfind('}');
     if (close != std::string::npos) rep = rep.substr(0, close) + (rep.size() > 2 ? ", " : "") + sw + graph + "}";

@@ -277,9 +277,10 @@ int launch_step_end(const View& v, cudaStream_t s, double warn, double err);
 int launch_rms(const View& v, cudaStream_t s, double* partial, double* out);
 int launch_scalar_begin(const View& v, cudaStream_t s);
 int launch_to_f32(const View& v, cudaStream_t s);
-// reference layout <-> SoA slots (dir 0: ref -> soa, dir 1: soa -> ref_out)
-int launch_ref_soa(const View& v, cudaStream_t s, int nk, int IX, int JX, const double* ref, double* soa,
-                   double* ref_out, int dir);
+// reference layout <-> SoA slots (dir 0: ref -> soa, dir 1: soa -> ref_out): the n cells
+// from the reference array's cell first on, whose values ref / ref_out hold
+int launch_ref_soa(const View& v, cudaStream_t s, int nk, int IX, int JX, long long first, long long n, const double* ref,
+                   double* soa, double* ref_out, int dir);
 
 // block sharding (k_shard.cu): exchange of the cells other ranks' ghost
 // copies read, and the device halves of the cross-rank reductions
