@@ -84,7 +84,8 @@ constexpr int kThreads = 256; // of a sweep CTA
 // warps by role: 0, 1 compute (on sub-partitions 0 and 1); the record loads and the
 // hand-off wait on sub-partitions 2 and 3, away from them
 constexpr int kWarpLoad = 2, kWarpIn = 4, kWarpOut = 6;
-constexpr long long kSpin = 1ll << 22;
+constexpr long long kSpin = 1ll << 22;   // polls of a wait
+constexpr long long kDrain = 1ll << 17;  // cycles (70 us)
 
 // hand-off chunks of a strip's top row for a plane of ni columns: chunk j
 // holds the columns 4j-3 .. 4j (HK = 4), j = 0 .. (ni + 2) / 4
@@ -941,6 +942,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_wave(View v, WaveArgs a) {
         }
         cluster_sync();  // the task is done in every CTA of the cluster
     }
+    // Where every wait came true, every chunk copied into this CTA's rings has been waited for.
+    // After one that gave up, chunks may still be on their way: their copies end (within a
+    // microsecond) before any CTA of the cluster leaves.
+    if (*reinterpret_cast<volatile int*>(s_bail) != 0)
+        for (const long long t0 = clock64(); clock64() - t0 < kDrain;) {
+        }
     cluster_sync();  // no CTA leaves while a peer may still reach its shared memory
 }
 

@@ -29,3 +29,12 @@ def test_dynamic_shared_memory_is_declared_aligned():
                 found += 1
                 assert re.search(r"__align__\((16|32|64|128)\)", decl), (name, decl)
     assert found >= 7
+
+
+def test_sweep_winds_down_with_its_copies():
+    """A sweep CTA whose wait gave up stays until the bulk copies on their way into its
+    shared memory have landed: that pause stands before the cluster's last barrier."""
+    src = source("k_wave.cu")
+    kernel = src[src.index("k_wave(View v, WaveArgs a)"):src.index("records_to_tile(")]
+    tail = kernel[kernel.rindex("cluster_sync();", 0, kernel.rindex("cluster_sync();")):]
+    assert re.search(r"\*s_bail\b|s_bail\) != 0", tail) and "kDrain" in tail
