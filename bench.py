@@ -120,7 +120,10 @@ def algo_bytes(kind, case, mixed):
         geo = 28 if case.desc.viscous else 14
         return wb * (W + nY) + 8 * ((3 * D if nr else 2 * D) + geo + D + 3)
     if kind in (abi.K_SWEEP_FWD, abi.K_SWEEP_BWD):
-        return 8 * (D + 1 + 4 + 2 * nY + 2 + 4 + 2 + 1 + D)
+        # the strip records as they lie (k_wave.cu): read whole, the X part written back.
+        # One species: X 4, own coefficients 16, shared 20 a cell; 8 and 9: 12, 24, 16
+        read, written = (40, 4) if nY == 1 else (52, 12)
+        return wb * (read + written)
     if kind == abi.K_UPDATE:
         # NR: k_omega (Dq of the species and energy, q of the species) and k_unpack
         # (q += omega Dq), averaged over the two launches

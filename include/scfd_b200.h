@@ -273,7 +273,12 @@ int  scfd_profile(scfd_ctx* ctx, int enable);
  * restored after) and the fastest is kept; the candidates compute the same
  * values.  SCFD_AUTOTUNE=0 in the environment keeps the default shapes;
  * SCFD_RES_TILE=<k> pins the residual to tile k of the list (e.g. to profile
- * one shape). */
+ * one shape).  The object also gives the sweeps (kind, tasks, clusters and CTAs per
+ * cluster, or for the generic sweeps the reason: SCFD_SWEEP_LEGACY is set, the
+ * species count has no wavefront, no cluster fits, the strip records do not), the
+ * bytes of the arena and of the staging of host copies, and the steps of a graph
+ * once there is one.  SCFD_SWEEP_CLUSTER=8 takes the portable cluster size;
+ * SCFD_MEM_LIMIT=<bytes> commits as on a device with no more than that. */
 int  scfd_tuning(scfd_ctx* ctx, char* json, int len);
 int  scfd_kernel_stats(scfd_ctx* ctx, int kind, double* total_ms, int64_t* launches, char* name, int namelen);
 

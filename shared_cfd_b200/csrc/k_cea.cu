@@ -1060,8 +1060,8 @@ int cea_launch(scfd_cea* h, int64_t ncell, const double* rho, const double* Y, c
         // (4099 cells 54 us with the 255 registers that 2 blocks per SM leave, 58 with
         // 3 blocks; 40 000 cells 70 us with 3; shared-memory vectors 68 and 77).
         // Above that the shared-memory vectors, whose small code and more resident warps
-        // win (2^17 cells 162 us against 192): 4 blocks per SM without spills, and 5 for four
-        // waves and more (2^20 cells 1093 us against 1133, and 1285 in registers).
+        // win (2^17 cells 162 us against 192): 4 blocks per SM with next to no spills, and 5 for
+        // four waves and more (2^20 cells 1095 us against 1133, and 1285 in registers).
         int dev = 0, nsm = 148;
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         if (blocks <= 2ll * nsm)

@@ -13,7 +13,9 @@
 // in FP64, 9.5 of 16 in FP32, with DRAM at a fifth of its rate).  So each phase issues all
 // its loads before it uses or stores any: a thread stages whole cells, W values in
 // flight at once, and reads q, qp, qpp of its cell before the first store; face fluxes lie
-// component-major.  786 k cells, 9 species: FP64 0.385 -> 0.301 ms, FP32 0.357 -> 0.216;
+// component-major (precond_cell, the cell phase of the preconditioned schemes, still
+// stores among its loads).  786 k cells, 9 species: FP64 0.385 -> 0.301-0.310 ms over three
+// GPUs, FP32 0.357 -> 0.216-0.221;
 // 197 k cells of one species FP64 (explicit) 0.035 -> 0.028 ms.  A 16x7 tile of 128 threads
 // (every round of faces full) was slower in FP64 (0.353 against 0.313 ms then).
 // The FP64 kernel stages w and T only and reads vhi through L1: its 16x8 tile

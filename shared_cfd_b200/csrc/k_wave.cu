@@ -15,7 +15,8 @@
 //
 // What bounds it: the chain of ni + nj dependent steps, and in each step the
 // issue and the dependence chain of one warp (about 2 cycles per FP64 or FP32
-// instruction, 4 per shuffle), not memory (DRAM at 3 %).  So a cell's D components
+// instruction, 4 per shuffle), not memory (786 k cells of 9 species FP64: 342 MB in
+// 269 us, 1.27 TB/s, 19 % of the copy rate).  So a cell's D components
 // are spread over four lanes, a plane's rows over all the SMs that the clusters
 // can have, and what is not the chain is taken off the step: the next step's
 // record is read into registers while this one is computed, results go straight to
