@@ -328,7 +328,10 @@ __device__ __forceinline__ void thermo_fixed(const View& v, long long c) {
     double T = div_pos(w[3 * N + c], rho * w[iR * N + c]);
     double kappa, MW, mu;
     const int st = dev_calc_T_fixed<NS>(v.chem, vrho, rho, ei, T, kappa, MW, DH, vh, mu);
-    if (st) set_status(v.sc, st);
+    if (st) {  // nothing was formed: the cell keeps what it had
+        set_status(v.sc, st);
+        return;
+    }
 #pragma unroll
     for (int k = 0; k < nY; ++k) {
         v.DHi[k * N + c] = DH[k];
@@ -380,7 +383,10 @@ __device__ __forceinline__ void thermo_any(const View& v, long long c) {
     double T = w[3 * N + c] / (rho * w[iR * N + c]);
     double kappa, MW, mu;
     const int st = dev_calc_T(v.chem, vrho, rho, ei, T, kappa, MW, DH, vh, mu);
-    if (st) set_status(v.sc, st);
+    if (st) {  // nothing was formed: the cell keeps what it had
+        set_status(v.sc, st);
+        return;
+    }
     for (int k = 0; k < nY; ++k) {
         v.DHi[k * N + c] = DH[k];
         v.vhi[k * N + c] = vh[k];
